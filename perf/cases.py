@@ -45,15 +45,15 @@ RANGES = {
 # below); one right-hand side takes about 143 and one analytical Jacobian 273
 # FP64 operations per reaction (drm19: 12,023 and 22,908).
 COUNTS = {
-    "react": (46.5, 1.05, 8.7, 43.5),
-    "react loose": (20.0, 1.0, 5.0, 17.0),
-    "box": (310.0, 5.0, 40.0, 300.0),
-    "large": (22.6, 1.0, 7.3, 19.6),
-    "heptane": (47.3, 1.07, 10.7, 44.3),
-    "qss": (44.0, 0.0, 9.0, 41.0),
-    "srk": (350.0, 0.0, 40.0, 340.0),
-    "adjoint": (60.0, 1.5, 10.0, 55.0),
-    "arkode": (311.0, 0.0, 0.0, 0.0),
+    "react": (54.6, 1.09, 9.8, 51.6),
+    "react loose": (17.9, 1.0, 5.4, 14.9),
+    "box": (826.0, 14.8, 79.1, 823.6),
+    "large": (38.0, 1.0, 9.7, 35.0),
+    "heptane": (46.7, 1.07, 10.7, 43.7),
+    "qss": (57.8, 0.0, 8.4, 40.7),  # the difference quotients' right-hand sides among the first
+    "srk": (588.6, 0.0, 56.4, 496.7),
+    "adjoint": (69.3, 1.24, 11.8, 66.3),
+    "arkode": (321.0, 0.0, 0.0, 0.0),
 }
 
 
