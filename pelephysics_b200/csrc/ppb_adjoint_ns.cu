@@ -97,18 +97,20 @@ __device__ __forceinline__ SegTape seg_tape(const AdjCells& C, int c, int n)
           C.yinfo + (size_t)c * C.cap_y * 2};
 }
 
-template <int NS, typename LT, typename B>
-__device__ __noinline__ void save_cp(const Team<32>& tm, char* dst, const B& bdf, const Work<LT>& w, int nstloc)
+// The integrator state and the workspace go by value: by reference they would
+// live in local memory for the whole recording loop.
+template <int NS, typename LT>
+__device__ __noinline__ void save_cp(Team<32> tm, char* dst, BdfScalars s, Work<LT> w, int nstloc)
 {
   constexpr int n = NS + 1;
   if (tm.lane == 0) {
-    *reinterpret_cast<BdfScalars*>(dst) = bdf.s;
-    *reinterpret_cast<BdfArrays*>(dst + sizeof(BdfScalars)) = bdf.ar;
+    *reinterpret_cast<BdfScalars*>(dst) = s;
+    *reinterpret_cast<BdfArrays*>(dst + sizeof(BdfScalars)) = *w.ba;
     *cp_tail(dst) = CpTail{nstloc, 0, 0, 0, -1};
   }
   double* z = reinterpret_cast<double*>(dst + cp_head_bytes<LT>());
   for (int j = 0; j < 6; j++)
-    for (int i = tm.lane; i < n; i += 32) z[j * n + i] = w.zn[j][i];
+    for (int i = tm.lane; i < n; i += 32) z[j * n + i] = w.zn[j * n + i];
   for (int i = tm.lane; i < n; i += 32) z[6 * n + i] = w.ewt[i];
   double* J = z + 7 * n;
   for (int i = tm.lane; i < n * n; i += 32) J[i] = w.J[i];
@@ -119,20 +121,26 @@ __device__ __noinline__ void save_cp(const Team<32>& tm, char* dst, const B& bdf
   tm.sync();
 }
 
-template <int NS, typename LT, typename B>
-__device__ __noinline__ void restore_cp(const Team<32>& tm, const char* src, B& bdf, Work<LT>& w, int& nstloc)
+struct CpScalars {
+  BdfScalars s;
+  int nstloc;
+};
+
+template <int NS, typename LT>
+__device__ __noinline__ CpScalars restore_cp(Team<32> tm, const char* src, Work<LT> w)
 {
   constexpr int n = NS + 1;
-  bdf.s = *reinterpret_cast<const BdfScalars*>(src);
+  CpScalars out;
+  out.s = *reinterpret_cast<const BdfScalars*>(src);
   {
     const double* a = reinterpret_cast<const double*>(src + sizeof(BdfScalars));
     for (int i = tm.lane; i < (int)(sizeof(BdfArrays) / sizeof(double)); i += 32)
-      reinterpret_cast<double*>(&bdf.ar)[i] = a[i];
+      reinterpret_cast<double*>(w.ba)[i] = a[i];
   }
-  nstloc = cp_tail(src)->nstloc;
+  out.nstloc = cp_tail(src)->nstloc;
   const double* z = reinterpret_cast<const double*>(src + cp_head_bytes<LT>());
   for (int j = 0; j < 6; j++)
-    for (int i = tm.lane; i < n; i += 32) w.zn[j][i] = z[j * n + i];
+    for (int i = tm.lane; i < n; i += 32) w.zn[j * n + i] = z[j * n + i];
   for (int i = tm.lane; i < n; i += 32) w.ewt[i] = z[6 * n + i];
   const double* J = z + 7 * n;
   for (int i = tm.lane; i < n * n; i += 32) w.J[i] = (LT)J[i];
@@ -141,7 +149,8 @@ __device__ __noinline__ void restore_cp(const Team<32>& tm, const char* src, B& 
   const int* piv = reinterpret_cast<const int*>(A + n * n);
   for (int i = tm.lane; i < n; i += 32) w.piv[i] = piv[i];
   tm.sync();
-  perm_from_piv(tm, w.piv, w.perm, n);
+  solve_prep<32, LT>(tm, w.A, w.piv, w.perm, w.dinv, n);
+  return out;
 }
 
 // Pointwise: f, df/dy, df/dE and, for a weight vector v per cell,
@@ -231,7 +240,7 @@ static int launch_rhs_exact_ns(const DevMech& M, int rtype, double t, const doub
 // Copy a just-recorded segment (records, states, their (t, gamma)) into the
 // next free bytes of the tape pool and note where in its checkpoint's tail;
 // when the pool is full the segment is recomputed in the reverse sweep.
-static __device__ __noinline__ void copy_segment(const Team<32>& tm, const AdjCells& C, char* cp, const TapeRec* tape,
+static __device__ __noinline__ void copy_segment(Team<32> tm, const AdjCells& C, char* cp, const TapeRec* tape,
                                                  const double* ys, const double* yinfo, int nrec, int ny, int n)
 {
   size_t yo, io;
@@ -273,8 +282,7 @@ enum : int { SEG_FORWARD = 0, SEG_REPLAY = 1, SEG_TANGENT = 2 };
 // warp) swept forward by the tangent-linear model as soon as it is recorded;
 // dy(t_end) goes to b.lam_y0.  Needs the adjoint workspace after the
 // integrator's in each warp's shared memory.
-// All modes share the one call site of start() and of advance(), so every
-// mode integrates with the same compiled arithmetic and their trajectories
+// All modes share the one call site of the integrator (drive), so every mode integrates with the same compiled arithmetic and their trajectories
 // agree bit for bit.
 template <int NS, typename LT>
 __global__ void __launch_bounds__(512, 1) k_adj_seg(const __grid_constant__ DevMech M, const __grid_constant__ Options o,
@@ -322,55 +330,33 @@ __global__ void __launch_bounds__(512, 1) k_adj_seg(const __grid_constant__ DevM
       w.src[i] = (i < NS && b.src) ? b.src[(size_t)c * NS + i] : 0.0;
       if (o.use_typ_vals) w.atolv[i] = b.atolv[i];
       if (!replay) {
-        w.zn[0][i] = y0[i];
+        w.zn[i] = y0[i];
         w.y[i] = y0[i];
       }
     }
     tm.sync();
     const CellIn cin{b.rhoe[c], b.rhoesrc ? b.rhoesrc[c] : 0.0};
-    Bdf<NS, 32, LT, AdjRec<32>> bdf(tm, M, o, w, cin);
+    AdjRec<32> rec;
+    Bdf<NS, 32, LT, AdjRec<32>> bdf(tm, M, o, w, cin, rec);
     const size_t slot_t = tangent ? gwarp : (size_t)c; // the tape's owner
     TapeRec* tape = reinterpret_cast<TapeRec*>(C.tape) + slot_t * C.cap_rec;
     double* ys = C.ys + slot_t * C.cap_y * n;
-    bdf.rec.tape = tape;
-    bdf.rec.ys = ys;
-    bdf.rec.yinfo = (tangent || !C.yinfo) ? nullptr : C.yinfo + (size_t)c * C.cap_y * 2;
-    bdf.rec.n = n;
-    bdf.rec.seg_steps = C.seg_steps;
-    bdf.rec.close_rec = C.close_rec;
-    bdf.rec.close_y = C.close_y;
-    bdf.rec.begin();
+    rec.tape = tape;
+    rec.ys = ys;
+    rec.yinfo = (tangent || !C.yinfo) ? nullptr : C.yinfo + (size_t)c * C.cap_y * 2;
+    rec.n = n;
+    rec.seg_steps = C.seg_steps;
+    rec.close_rec = C.close_rec;
+    rec.close_y = C.close_y;
+    rec.begin();
     AdjSweep<32, (NS + 31) / 32, LT> sw{tm, M, o, w, a, cin, n, o.max_order};
     const double dE = (tangent && b.dE) ? b.dE[c] : 0.0;
     int nstloc = 0, ncp = 0, flag = ST_OK;
     bool done = false;
     int* cpi = C.cp_idx + (size_t)c * C.max_seg;
-    if (!replay) {
-      flag = bdf.start(dt);
-      if (tangent) {
-        for (int i = tm.lane; i < 6 * n; i += 32) a.lam[i] = 0.0;
-        for (int i = tm.lane; i < n; i += 32) a.pend[i] = 0.0;
-        tm.sync();
-        if (flag == ST_OK) {
-          // z_0 = y0, z_1 = h0 f(0, y0)
-          for (int i = tm.lane; i < n; i += 32) a.lam[i] = b.dy0 ? b.dy0[(size_t)c * n + i] : 0.0;
-          tm.sync();
-          sw.fwd_freset(0.0, bdf.rec.h0, y0, dE, b.dp);
-        }
-      } else {
-        for (int i = tm.lane; i < 7 * n; i += 32) C.lam[(size_t)c * 7 * n + i] = 0.0;
-        for (int r = tm.lane; r < 3 * R; r += 32) C.gw[(size_t)c * 3 * R + r] = 0.0;
-        if (b.lam_y0)
-          for (int i = tm.lane; i < n; i += 32) b.lam_y0[(size_t)c * n + i] = 0.0;
-        if (tm.lane == 0) {
-          C.lamE[c] = 0.0;
-          if (b.lam_e) b.lam_e[c] = 0.0;
-        }
-      }
-    }
-    for (;;) {
-      if (flag != ST_OK) break;
-      if (mode == SEG_FORWARD) {
+    // one call site of the integrator: first its start, then segment by segment
+    for (bool fresh = !replay;; fresh = false) {
+      if (!fresh && mode == SEG_FORWARD) {
         if (ncp >= C.max_seg) {
           flag = ST_ADJ_CAPACITY;
           break;
@@ -383,22 +369,47 @@ __global__ void __launch_bounds__(512, 1) k_adj_seg(const __grid_constant__ DevM
           break;
         }
         if (tm.lane == 0) cpi[ncp] = slot;
-        save_cp<NS, LT>(tm, C.cp_pool + (size_t)slot * C.cp_stride, bdf, w, nstloc);
+        save_cp<NS, LT>(tm, C.cp_pool + (size_t)slot * C.cp_stride, bdf.s, w, nstloc);
         ncp++;
       } else if (replay) {
-        restore_cp<NS, LT>(tm, C.cp_pool + (size_t)cpi[seg] * C.cp_stride, bdf, w, nstloc);
+        const CpScalars cs = restore_cp<NS, LT>(tm, C.cp_pool + (size_t)cpi[seg] * C.cp_stride, w);
+        bdf.s = cs.s;
+        nstloc = cs.nstloc;
       }
-      bdf.rec.begin();
-      flag = bdf.advance(dt, nstloc, done);
-      if (tangent && flag == ST_OK) flag = sw.forward(tape, bdf.rec.nrec, ys, dE, b.dp, a.tmp);
+      rec.begin();
+      flag = bdf.drive(dt, nstloc, done, fresh);
+      if (fresh) {
+        if (tangent) {
+          for (int i = tm.lane; i < 6 * n; i += 32) a.lam[i] = 0.0;
+          for (int i = tm.lane; i < n; i += 32) a.pend[i] = 0.0;
+          tm.sync();
+          if (flag == ST_OK) {
+            // z_0 = y0, z_1 = h0 f(0, y0)
+            for (int i = tm.lane; i < n; i += 32) a.lam[i] = b.dy0 ? b.dy0[(size_t)c * n + i] : 0.0;
+            tm.sync();
+            sw.fwd_freset(0.0, rec.h0, y0, dE, b.dp);
+          }
+        } else {
+          for (int i = tm.lane; i < 7 * n; i += 32) C.lam[(size_t)c * 7 * n + i] = 0.0;
+          for (int r = tm.lane; r < 3 * R; r += 32) C.gw[(size_t)c * 3 * R + r] = 0.0;
+          if (b.lam_y0)
+            for (int i = tm.lane; i < n; i += 32) b.lam_y0[(size_t)c * n + i] = 0.0;
+          if (tm.lane == 0) {
+            C.lamE[c] = 0.0;
+            if (b.lam_e) b.lam_e[c] = 0.0;
+          }
+        }
+        if (flag != ST_OK) break;
+        continue;
+      }
+      if (tangent && flag == ST_OK) flag = sw.forward(tape, rec.nrec, ys, dE, b.dp, a.tmp);
       if (mode == SEG_FORWARD && flag == ST_OK && !done && C.tpool)
-        copy_segment(tm, C, C.cp_pool + (size_t)cpi[ncp - 1] * C.cp_stride, tape, ys, bdf.rec.yinfo, bdf.rec.nrec,
-                     bdf.rec.ny, n);
+        copy_segment(tm, C, C.cp_pool + (size_t)cpi[ncp - 1] * C.cp_stride, tape, ys, rec.yinfo, rec.nrec, rec.ny, n);
       if (flag != ST_OK || done || replay) break;
     }
     if (!replay) {
       if (b.y_out)
-        for (int i = tm.lane; i < n; i += 32) b.y_out[(size_t)c * n + i] = (flag == ST_OK) ? w.y[i] : w.zn[0][i];
+        for (int i = tm.lane; i < n; i += 32) b.y_out[(size_t)c * n + i] = (flag == ST_OK) ? w.y[i] : w.zn[i];
       if (tangent && b.lam_y0)
         for (int i = tm.lane; i < n; i += 32) b.lam_y0[(size_t)c * n + i] = (flag == ST_OK) ? a.tmp[i] : 0.0;
       if (tm.lane == 0) {
@@ -415,9 +426,9 @@ __global__ void __launch_bounds__(512, 1) k_adj_seg(const __grid_constant__ DevM
         }
         if (!tangent) {
           C.nseg[c] = (flag == ST_OK) ? ncp : 0;
-          C.h0[c] = bdf.rec.h0;
-          C.nrec[c] = bdf.rec.nrec;
-          C.ny[c] = bdf.rec.ny;
+          C.h0[c] = rec.h0;
+          C.nrec[c] = rec.nrec;
+          C.ny[c] = rec.ny;
           if (C.toff) C.toff[c] = -1; // the last segment stays in the cell's own area
         }
       }
@@ -434,8 +445,8 @@ __global__ void __launch_bounds__(512, 1) k_adj_seg(const __grid_constant__ DevM
           C.nrec[c] = 0;
           C.ny[c] = 0;
         } else {
-          C.nrec[c] = bdf.rec.nrec;
-          C.ny[c] = bdf.rec.ny;
+          C.nrec[c] = rec.nrec;
+          C.ny[c] = rec.ny;
           if (C.toff) C.toff[c] = -1;
         }
       }

@@ -22,7 +22,7 @@ namespace ppb {
 // Optional per-phase cycle counters (compile with -DPPB_PHASE_TIMERS): each
 // team accumulates clock64() deltas per phase and adds them to
 // g_phase_cycles at the end of a cell.  Off in the shipped library.
-enum Phase { PH_RHS = 0, PH_JAC, PH_LU, PH_SOLVE, PH_NEWTON, PH_STEP, PH_TOTAL, PH_COUNT };
+enum Phase { PH_RHS = 0, PH_JAC, PH_LU, PH_SOLVE, PH_TOTAL, PH_COUNT };
 #ifdef PPB_PHASE_TIMERS
 static __device__ unsigned long long g_phase_cycles[PH_COUNT]; // one copy per translation unit
 #define PPB_TIC(ph) const long long _tic_##ph = clock64()
@@ -59,7 +59,8 @@ inline int rendezvous_bound(int cycles, int warps)
 // Team-shared per-cell workspace.  LT is the LU storage type.
 template <typename LT>
 struct Work {
-  double* zn[6];
+  double* zn;   // Nordsieck array: 6 rows of n (one pointer: an array of pointers indexed by order at
+                // run time keeps the whole struct in local memory and its pointers generic)
   double *ewt, *acor, *y, *tempv, *ftemp, *delta;
   double *src, *atolv;
   LT* J;        // saved Jacobian (the factor's precision)
@@ -68,6 +69,7 @@ struct Work {
   LT* A;
   int* piv;
   int* perm;  // row order of the factored matrix: row i of PA is row perm[i] of A
+  double* dinv; // reciprocals of the factor's diagonal (dinv[0] NaN: not usable, see quotient)
   struct BdfArrays* ba; // the integrator's coefficient arrays (team-shared)
   // rate scratch
   double *Y, *sc, *g, *qd, *wdot, *ei, *h1, *h2, *h3;
@@ -151,58 +153,64 @@ __device__ __forceinline__ void rendezvous_resume(int* rv)
 // QSS: a QSS mechanism (sc and g then have its QSS slots, qco the QSS
 // solve's scratch; the team path solves the QSS concentrations only when
 // QSS is set, the one-lane path whenever the mechanism has QSS species).
-template <int TEAM, bool QSS = false>
-__device__ double reactor_rhs(
+template <int TEAM, bool QSS = false, int NS = 0>
+__device__ __forceinline__ double reactor_rhs(
   const Team<TEAM>& tm, const DevMech& M, int rtype, double t, const double* y, double* ydot, double rhoe,
   double rhoesrc, const double* src, double* Y, double* sc, double* g, double* qd, double* wdot, double* ei,
-  double* qco = nullptr)
+  double* qco = nullptr, bool unrounded_e = false)
 {
-  const int N = M.nsp;
+  const int N = NS > 0 ? NS : M.nsp;
   double a = 0.0;
   for (int s = tm.lane; s < N; s += TEAM) a += y[s];
   const double rho = tm.sum(a);
   const double rinv = 1.0 / rho;
   for (int s = tm.lane; s < N; s += TEAM) Y[s] = y[s] * rinv;
-  tm.sync();
+  if constexpr (!(NS > 0 && NS <= TEAM)) tm.sync(); // (one species per lane: a lane reads its own)
   const double nrg = (rhoe + rhoesrc * t) * rinv;
   double T = y[N];
   const int EH = (rtype == 2);
-  t_from_energy(tm, M, EH, nrg, Y, T);
+  ThermoAtT at;
+  const EnergyProduct ep{rhoe + rhoesrc * t, rinv, unrounded_e};
+  t_from_energy<TEAM, NS>(tm, M, EH, nrg, Y, T, &at, &ep);
   const double invT = 1.0 / T;
   const double RT = RU * T;
   RateScratch rs{sc, g, qd, nullptr, qco};
+  const double* te = EH ? M.th_h : M.th_u;
   double cv;
   if constexpr (TEAM > 1) {
     // one pass over the species at the final T: the heat capacity (as
-    // mix_c), the energies, the concentrations, their sum and g/RT (as
-    // productionRate forms them), then the two sums together
+    // mix_c; the T solve's last iterate has it), the energies (for one
+    // species per lane, the T solve's too), the concentrations, their sum
+    // and g/RT (as productionRate forms them)
+    constexpr bool ONE = NS > 0 && NS <= TEAM;
     const double logT = ppb_log(T);
     const double refC = 101325 / 8.31446 * invT;
     const double refCinv = 1 / refC;
-    double cvs = 0.0, mix = 0.0;
+    double mix = 0.0;
     for (int s = tm.lane; s < N; s += TEAM) {
       const double im = __ldg(M.imw + s);
-      cvs += Y[s] * (EH ? cp_R(M, s, T) : cv_R(M, s, T)) * __ldg(M.imw + s);
-      ei[s] = (EH ? h_RT(M, s, T, invT) : u_RT(M, s, T, invT)) * (RT * im);
+      double el = at.e;
+      if (!(ONE && at.have)) el = e_RT<NS>(M, te, s, T, invT);
+      ei[s] = el * (RT * im);
       const double scs = (rho * Y[s] * im) * 1.0e6;
       sc[s] = scs;
       mix += scs;
-      g[s] = g_RT(M, s, T, invT, logT);
+      g[s] = g_RT<NS>(M, s, T, invT, logT);
     }
-    cv = tm.sum(cvs) * RU;
     const double mixture = tm.sum(mix);
+    cv = at.have ? at.csum * RU : mix_c(tm, M, EH, T, Y);
     if (tm.lane == 0) {
       sc[N] = 1.0; // padding slots of the packed reaction records
       g[N] = 0.0;
     }
     tm.sync();
     if constexpr (QSS) qss_solve<TEAM>(tm, M, sc, g, T, invT, logT, refC, refCinv, mixture, qco, qco + 2 * M.nrq);
-    production_rate_core(tm, M, wdot, sc, T, invT, logT, refC, refCinv, mixture, rs);
+    production_rate_core<TEAM, NS>(tm, M, wdot, sc, T, invT, logT, refC, refCinv, mixture, rs);
   } else {
     cv = mix_c(tm, M, EH, T, Y);
     for (int s = tm.lane; s < N; s += TEAM) {
       const double im = __ldg(M.imw + s);
-      ei[s] = (EH ? h_RT(M, s, T, invT) : u_RT(M, s, T, invT)) * (RT * im);
+      ei[s] = e_RT(M, te, s, T, invT) * (RT * im);
       sc[s] = (rho * Y[s] * im) * 1.0e6;
     }
     if (tm.lane == 0) sc[N] = 1.0; // padding slot of the packed reaction records
@@ -281,7 +289,7 @@ __device__ double reactor_rhs_srk(
 
 // Reactor Jacobian, column-major n x n: J[i*n + k] = d f_k / d y_i.
 template <int TEAM, int PER>
-__device__ void reactor_jac(
+__device__ __noinline__ void reactor_jac(
   const Team<TEAM>& tm, const DevMech& M, int rtype, const double* y, double* J, double* sc, double* g,
   double* wdot, double* h1, double* h2, double* h3, double* h4, double* qd = nullptr, double* jx = nullptr)
 {
@@ -315,106 +323,260 @@ __device__ void reactor_jac(
 
 // ---------------------------------------------------------------- dense LU
 // Partial-pivoting LU of a column-major n x n matrix (first maximum wins, as
-// the SUNDIALS dense GETRF).  Returns 0 or k+1 for a zero pivot.
-template <int TEAM, typename LT>
-__device__ int lu_factor(const Team<TEAM>& tm, LT* A, int n, int* piv)
+// the SUNDIALS dense GETRF), one thread.  Returns 0 or k+1 for a zero pivot;
+// an all-NaN column counts as zero.
+template <typename LT>
+__device__ int lu_factor(LT* A, int n, int* piv)
 {
   for (int k = 0; k < n; k++) {
     LT* colk = A + k * n;
-    if constexpr (TEAM == 32) {
-      if (n - k <= 32) {
-        // one row per lane (row k + lane): the largest magnitude by a max
-        // reduction, the first row holding it by a ballot (rows in lane
-        // order), its value by one shuffle, so the reciprocal overlaps the
-        // row swap; a NaN entry never wins (its lane stays at -1)
-        const int i = k + tm.lane;
-        const LT a = i < n ? colk[i] : (LT)0;
-        const double v = fabs((double)a);
-        const double mine = (i < n && v > -1.0) ? v : -1.0;
-        double mx = mine;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const unsigned hit = __ballot_sync(0xffffffffu, i < n && mine == mx);
-        const int src = hit ? __ffs(hit) - 1 : 0;
-        const LT pv = __shfl_sync(0xffffffffu, a, src);
-        const int l = k + src;
-        if (!(mx > 0.0) || !hit) {
-          tm.sync();
-          return k + 1;
-        }
-        if (tm.lane == 0) piv[k] = l;
-        const LT mult = (LT)1.0 / pv;
-        if (l != k) {
-          for (int j = tm.lane; j < n; j += TEAM) {
-            const LT t = A[j * n + l];
-            A[j * n + l] = A[j * n + k];
-            A[j * n + k] = t;
-          }
-        }
-        tm.sync();
-        if (i > k && i < n) {
-          // the lane scales its own row's multiplier and keeps it
-          const LT lik = colk[i] * mult;
-          colk[i] = lik;
-#pragma unroll 4
-          for (int j = k + 1; j < n; j++) {
-            const LT akj = A[j * n + k];
-            if (akj != (LT)0) A[j * n + i] -= akj * lik;
-          }
-        }
-        tm.sync();
-        continue;
-      }
-    }
     double best = -1.0;
-    int bi = n;
-    for (int i = k + tm.lane; i < n; i += TEAM) {
+    int l = n;
+    for (int i = k; i < n; i++) {
       const double v = fabs((double)colk[i]);
       if (v > best) {
         best = v;
-        bi = i;
+        l = i;
       }
     }
-    if constexpr (TEAM <= 32) {
-#pragma unroll
-      for (int o = TEAM / 2; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(tm.mask, best, o, TEAM);
-        const int oi = __shfl_xor_sync(tm.mask, bi, o, TEAM);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-    } else {
-      tm.argmax(best, bi);
-    }
-    const int l = bi;
-    // a zero column is singular; an all-NaN column selects no row (bi == n)
-    if (!(best > 0.0) || l >= n) {
-      tm.sync();
-      return k + 1;
-    }
-    if (tm.lane == 0) piv[k] = l;
+    if (!(best > 0.0)) return k + 1;
+    piv[k] = l;
     if (l != k) {
-      for (int j = tm.lane; j < n; j += TEAM) {
+      for (int j = 0; j < n; j++) {
         const LT t = A[j * n + l];
         A[j * n + l] = A[j * n + k];
         A[j * n + k] = t;
       }
     }
-    tm.sync();
     const LT mult = (LT)1.0 / colk[k];
-    for (int i = k + 1 + tm.lane; i < n; i += TEAM) colk[i] *= mult;
-    tm.sync();
-    for (int i = k + 1 + tm.lane; i < n; i += TEAM) {
+    for (int i = k + 1; i < n; i++) colk[i] *= mult;
+    for (int i = k + 1; i < n; i++) {
       const LT lik = colk[i];
       for (int j = k + 1; j < n; j++) {
         const LT akj = A[j * n + k];
         if (akj != (LT)0) A[j * n + i] -= akj * lik;
       }
     }
-    tm.sync();
   }
+  return 0;
+}
+
+// |a| as an unsigned pair (hi, lo) in the order of the magnitudes; 0 for a
+// NaN, which never becomes the pivot.
+__device__ __forceinline__ void pivot_key(double a, unsigned& hi, unsigned& lo)
+{
+  hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  lo = (unsigned)__double2loint(a);
+  if (!(a == a)) hi = lo = 0u;
+}
+__device__ __forceinline__ void pivot_key(float a, unsigned& hi, unsigned& lo)
+{
+  hi = a == a ? (__float_as_uint(a) & 0x7fffffffu) : 0u;
+  lo = 0u;
+}
+
+// x - u l where the pivot row's entry u is nonzero (else x, also against a
+// multiplier that is not finite): a select, no branch.
+template <typename LT>
+__device__ __forceinline__ LT lu_update(LT x, LT u, LT l)
+{
+  const LT v = x - u * l;
+  return u != (LT)0 ? v : x;
+}
+
+// The same factorisation by a team, every entry by the same operations in the
+// same order; perm gets the row order (row i of PA is row perm[i] of A).
+//
+// It is bound by the latency of the chain from one column to the next, so the
+// chain is kept short.  Lane r of a warp holds row k + r (+ 32, + 64) of
+// column k; the largest magnitude is found by integer max reductions over the
+// bits of |a| (one instruction each; two for FP64) and a ballot for the first
+// row holding it, where a butterfly of doubles takes five levels of two
+// shuffles and a compare.  The row swap is part of the update: a lane reads
+// the pivot row's entry and the displaced row's entry of each column it
+// updates and writes both back, so no pass and no barrier of its own.  With
+// 16 rows or fewer left, the lanes split into groups that take several
+// columns at a time.
+// Several warps: every warp finds the pivot by itself (no barrier) and owns
+// the columns j with j mod NW equal to its number, for the swap and the
+// update; column k itself, which every warp reads, is scaled by its owner
+// after the next column's barrier.  One barrier a column.
+// drm19 (22 x 22, one warp alone on its SM): 39,700 SM clocks before.
+template <int TEAM, typename LT, int RPL>
+__device__ __forceinline__ int lu_factor_team(const Team<TEAM>& tm, LT* A, int n, int* piv, int* perm)
+{
+  constexpr int W = Team<TEAM>::W, NW = Team<TEAM>::NW;
+  const int wl = tm.lane % W, wid = tm.lane / W;
+  const unsigned mask = tm.mask;
+  int pr[RPL]; // the row order: entries wl + W c
+  LT held[RPL]; // the scaled column the warp still has to write (NW > 1)
+  LT held_p = (LT)0;
+#pragma unroll
+  for (int c = 0; c < RPL; c++) {
+    pr[c] = wl + W * c;
+    held[c] = (LT)0;
+  }
+  for (int k = 0; k < n; k++) {
+    LT* colk = A + k * n;
+    if constexpr (NW > 1) {
+      __syncthreads(); // column k is final on every warp
+      if (k > 0 && wid == (k - 1) % NW) {
+        // the owner's scaled column k - 1
+        LT* cp = colk - n;
+#pragma unroll
+        for (int c = 0; c < RPL; c++) {
+          const int i = k - 1 + wl + W * c;
+          if (i > k - 1 && i < n) cp[i] = held[c];
+        }
+        if (wl == 0) cp[k - 1] = held_p;
+        __syncwarp();
+      }
+    }
+    // ---- the pivot
+    LT a[RPL];
+    unsigned hi[RPL], lo[RPL], bh = 0u, bl = 0u;
+#pragma unroll
+    for (int c = 0; c < RPL; c++) {
+      const int i = k + wl + W * c;
+      a[c] = i < n ? colk[i] : (LT)0;
+      pivot_key(a[c], hi[c], lo[c]);
+      if (hi[c] > bh || (hi[c] == bh && lo[c] > bl)) {
+        bh = hi[c];
+        bl = lo[c];
+      }
+    }
+    const unsigned mh = __reduce_max_sync(mask, bh);
+    unsigned ml = 0u;
+    if constexpr (sizeof(LT) == sizeof(double)) ml = __reduce_max_sync(mask, bh == mh ? bl : 0u);
+    if ((mh | ml) == 0u) { // zero (or NaN) column
+      tm.sync();
+      return k + 1;
+    }
+    int l = k;
+    LT pv = (LT)0;
+    bool found = false;
+#pragma unroll
+    for (int c = 0; c < RPL; c++) {
+      const unsigned hit = __ballot_sync(mask, hi[c] == mh && lo[c] == ml) >> (W < 32 ? (threadIdx.x & 31) / W * W : 0);
+      if (!found && hit) {
+        const int src = __ffs(hit) - 1;
+        l = k + src + W * c;
+        pv = __shfl_sync(mask, a[c], src, W);
+        found = true;
+      }
+    }
+    const LT ak = __shfl_sync(mask, a[0], 0, W); // the displaced row's entry
+    const LT mult = (LT)1.0 / pv;
+    if (tm.lane == 0) piv[k] = l;
+    if (l != k) { // row order
+      int pk = 0, pl = 0;
+#pragma unroll
+      for (int c = 0; c < RPL; c++) {
+        if (k / W == c) pk = __shfl_sync(mask, pr[c], k % W, W);
+        if (l / W == c) pl = __shfl_sync(mask, pr[c], l % W, W);
+      }
+#pragma unroll
+      for (int c = 0; c < RPL; c++) {
+        const int i = wl + W * c;
+        if (i == k) pr[c] = pl;
+        if (i == l) pr[c] = pk;
+      }
+    }
+    // ---- the multipliers of the lane's rows
+    LT lik[RPL];
+#pragma unroll
+    for (int c = 0; c < RPL; c++) lik[c] = (k + wl + W * c == l ? ak : a[c]) * mult;
+    // ---- the factor's earlier columns: the swap alone
+    if (l != k) {
+      for (int j = wid + NW * wl; j < k; j += NW * W) {
+        const LT t = A[j * n + k];
+        A[j * n + k] = A[j * n + l];
+        A[j * n + l] = t;
+      }
+    }
+    if constexpr (NW == 1) {
+#pragma unroll
+      for (int c = 0; c < RPL; c++) {
+        const int i = k + wl + W * c;
+        if (i == k) colk[i] = pv;
+        else if (i < n) colk[i] = lik[c];
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < RPL; c++) held[c] = lik[c];
+      held_p = pv;
+    }
+    // ---- swap and update of the later columns
+    if constexpr (NW == 1 && RPL == 1) {
+      const int m = n - 1 - k; // rows left
+      if (m > 0) {
+        const int s = m > 1 ? 32 - __clz(m - 1) : 0; // 2^s rows (or more) a group
+        const int G = W >> s, r = wl & ((1 << s) - 1), g = wl >> s;
+        const int i = k + 1 + r;
+        const LT lr = __shfl_sync(mask, lik[0], (1 + r) % W, W);
+        constexpr int U = 4;
+        for (int jb = k + 1; jb < n; jb += U * G) {
+          LT t[U], u[U], x[U];
+#pragma unroll
+          for (int q = 0; q < U; q++) {
+            const int j = jb + q * G + g;
+            const LT* cj = A + (j < n ? j : k) * n;
+            t[q] = cj[k];
+            u[q] = cj[l];
+            x[q] = cj[r < m ? i : k];
+          }
+          __syncwarp(mask);
+#pragma unroll
+          for (int q = 0; q < U; q++) {
+            const int j = jb + q * G + g;
+            LT* cj = A + j * n;
+            if (j < n && r < m) cj[i] = lu_update(i == l ? t[q] : x[q], u[q], lr);
+            if (j < n && r == 0) cj[k] = u[q];
+          }
+        }
+      }
+      __syncwarp(mask);
+    } else {
+      constexpr int U = 2;
+      // first column after k that the warp owns
+      int j0 = k + 1;
+      if constexpr (NW > 1) j0 += ((wid - j0) % NW + NW) % NW;
+      for (int jb = j0; jb < n; jb += U * NW) {
+        LT t[U], u[U], x[U][RPL];
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+          const int j = jb + q * NW;
+          const LT* cj = A + (j < n ? j : jb) * n;
+          t[q] = cj[k];
+          u[q] = cj[l];
+#pragma unroll
+          for (int c = 0; c < RPL; c++) {
+            const int i = k + wl + W * c;
+            x[q][c] = i < n ? cj[i] : (LT)0;
+          }
+        }
+        __syncwarp(mask);
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+          const int j = jb + q * NW;
+          LT* cj = A + j * n;
+#pragma unroll
+          for (int c = 0; c < RPL; c++) {
+            const int i = k + wl + W * c;
+            const LT v = lu_update(i == l ? t[q] : x[q][c], u[q], lik[c]);
+            if (j < n && i < n) cj[i] = i == k ? u[q] : v;
+          }
+        }
+      }
+      __syncwarp(mask);
+    }
+  }
+  if (wid == 0) {
+#pragma unroll
+    for (int c = 0; c < RPL; c++)
+      if (wl + W * c < n) perm[wl + W * c] = pr[c];
+  }
+  tm.sync();
   return 0;
 }
 
@@ -451,13 +613,37 @@ __device__ void lu_solve(const Team<TEAM>& tm, const LT* A, int n, const int* pi
   tm.sync();
 }
 
+// Reciprocals of a factor's diagonal, each one IEEE division; dinv[0] becomes
+// NaN when a diagonal entry is outside what quotient() covers.
+template <int TEAM, typename LT>
+__device__ __forceinline__ void diag_recip(const Team<TEAM>& tm, const LT* A, double* dinv, int n)
+{
+  bool ok = true;
+  for (int i = tm.lane; i < n; i += TEAM) {
+    const double a = (double)A[i * n + i];
+    const unsigned long long u = (unsigned long long)__double_as_longlong(a);
+    const unsigned e = (unsigned)(u >> 52) & 0x7ffu; // 2^-400 <= |a| <= 2^400, not all ones
+    ok = ok && (e - 623u <= 800u) && ((u & 0xfffffffffffffull) != 0xfffffffffffffull);
+    dinv[i] = 1.0 / a;
+  }
+  if constexpr (Team<TEAM>::NW > 1) {
+    ok = __syncthreads_and(ok) != 0;
+  } else {
+    ok = __all_sync(tm.mask, ok) != 0;
+    tm.sync();
+  }
+  if (!ok && tm.lane == 0) dinv[0] = __longlong_as_double(0x7ff8000000000000ll);
+  tm.sync();
+}
+
 // Row order of a factored matrix from its LAPACK-style pivots: the
 // interchanges k <-> piv[k], in order, applied to the identity, so that the
 // pivoted right-hand side is b[perm[0..n-1]].  A pivot outside [0, n) (pivots
 // of no factorisation yet, e.g. a checkpoint taken before the first step) is
-// skipped, so perm is always a permutation of 0..n-1.
-template <int TEAM>
-__device__ __forceinline__ void perm_from_piv(const Team<TEAM>& tm, const int* piv, int* perm, int n)
+// skipped, so perm is always a permutation of 0..n-1.  With it the
+// reciprocals of the diagonal.
+template <int TEAM, typename LT>
+__device__ __noinline__ void solve_prep(Team<TEAM> tm, const LT* A, const int* piv, int* perm, double* dinv, int n)
 {
   if (tm.lane == 0) {
     for (int i = 0; i < n; i++) perm[i] = i;
@@ -470,37 +656,108 @@ __device__ __forceinline__ void perm_from_piv(const Team<TEAM>& tm, const int* p
       }
     }
   }
-  tm.sync();
+  diag_recip(tm, A, dinv, n);
 }
 
-// lu_solve for a team of 16 or 32 lanes and n <= TEAM with the solution in
-// registers, lane i holding entry i: the pivoted gather, then the two
-// triangular sweeps with the running entry k broadcast by a shuffle instead of
-// a shared-memory round trip and a team barrier per column.  Every entry is
-// updated by the same operations in the same order as in lu_solve.
-template <int TEAM, typename LT, int NN>
-__device__ __forceinline__ void lu_solve_reg(const Team<TEAM>& tm, const LT* A, const int* perm, double* b)
+// The correctly rounded quotient b / a from y = 1 / a rounded (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990, theorem on the final step of a
+// division: with y correctly rounded, a's significand not all ones and q
+// within one ulp, q + y (b - a q) rounds to b / a).  The first correction
+// brings b y, up to two ulps off, within one.  Exact remainders need b, a and
+// the quotient away from the ends of the exponent range: the callers check b
+// and solve_prep a.  Five dependent operations where the inlined division
+// takes about twice that, a branch and an out-of-line slow path.
+__device__ __forceinline__ double quotient(double b, double a, double y)
 {
-  static_assert((TEAM == 16 || TEAM == 32) && NN <= TEAM, "one entry per lane");
-  const int i = tm.lane;
-  double x = (i < NN) ? b[perm[i]] : 0.0;
+  double q = b * y;
+  q = __fma_rn(__fma_rn(-a, q, b), y, q);
+  return __fma_rn(__fma_rn(-a, q, b), y, q);
+}
+
+// lu_solve out of line, for what quotient() does not cover.
+template <int TEAM, typename LT>
+__device__ __noinline__ void lu_solve_div(Team<TEAM> tm, const LT* A, int n, const int* piv, double* b)
+{
+  lu_solve<TEAM, LT>(tm, A, n, piv, b);
+}
+
+// lu_solve by the team's first warp with the solution in registers, lane r
+// holding entries r, r + W, ...: the pivoted gather, then the two triangular
+// sweeps with the running entry k broadcast by a shuffle instead of a
+// shared-memory round trip and a team barrier per column.  Every entry is
+// updated by the same operations in the same order as in lu_solve.
+// The sweeps are loops: unrolled over all columns, with a division each, they
+// were a third of the code a Newton iteration runs through, in a kernel bound
+// by instruction fetch.
+template <int TEAM, typename LT, int NN>
+__device__ __forceinline__ void lu_solve_reg(const Team<TEAM>& tm, const LT* A, const int* piv, const int* perm,
+                                             const double* dinv, double* b)
+{
+  constexpr int W = Team<TEAM>::W, NW = Team<TEAM>::NW, RPL = (NN + W - 1) / W;
+  const int wl = tm.lane % W;
+  double x[RPL];
+  bool bad = false;
+  if (NW == 1 || tm.lane < W) {
+    const double y0 = dinv[0];
+    bad = !(y0 == y0);
 #pragma unroll
-  for (int k = 0; k < NN - 1; k++) {
-    const double bk = __shfl_sync(tm.mask, x, k, TEAM);
-    if (i > k && i < NN) x -= (double)A[k * NN + i] * bk;
-  }
+    for (int c = 0; c < RPL; c++) x[c] = wl + W * c < NN ? b[perm[wl + W * c]] : 0.0;
 #pragma unroll
-  for (int k = NN - 1; k > 0; k--) {
-    const double bk = __shfl_sync(tm.mask, x, k, TEAM) / (double)A[k * NN + k];
-    if (i == k) {
-      x = bk;
-    } else if (i < k) {
-      x -= (double)A[k * NN + i] * bk;
+    for (int kb = 0; kb < RPL; kb++) {
+      const int k1 = kb < RPL - 1 ? W : NN - 1 - W * kb;
+#pragma unroll 3
+      for (int kk = 0; kk < k1; kk++) {
+        const int k = W * kb + kk;
+        const double bk = __shfl_sync(tm.mask, x[kb], kk, W);
+#pragma unroll
+        for (int c = kb; c < RPL; c++) {
+          const int i = wl + W * c;
+          const double a = (double)A[k * NN + (i < NN ? i : 0)];
+          if (i > k && i < NN) x[c] -= a * bk;
+        }
+      }
+    }
+#pragma unroll
+    for (int kb = RPL - 1; kb >= 0; kb--) {
+      const int k1 = kb < RPL - 1 ? W : NN - W * kb;
+#pragma unroll 3
+      for (int kk = k1 - 1; kk >= 0; kk--) {
+        const int k = W * kb + kk;
+        const double b0 = __shfl_sync(tm.mask, x[kb], kk, W);
+        const double bk = quotient(b0, (double)A[k * NN + k], dinv[k]);
+        // |b| within 2^-500 .. 2^500, or zero
+        const unsigned e = ((unsigned)__double2hiint(b0) >> 20) & 0x7ffu;
+        bad = bad || (e - 523u > 1000u && b0 != 0.0);
+#pragma unroll
+        for (int c = 0; c <= kb; c++) {
+          const int i = wl + W * c;
+          const double a = (double)A[k * NN + (i < NN ? i : 0)];
+          if (i == k) {
+            x[c] = bk;
+          } else if (i < k) {
+            x[c] -= a * bk;
+          }
+        }
+      }
     }
   }
-  if (i == 0) x /= (double)A[0];
-  tm.sync(); // every lane has gathered its entry before any writes
-  if (i < NN) b[i] = x;
+  if constexpr (NW > 1) {
+    bad = __syncthreads_or(bad) != 0;
+  } else {
+    bad = __any_sync(tm.mask, bad) != 0;
+  }
+  if (bad) {
+    lu_solve_div<TEAM, LT>(tm, A, NN, piv, b);
+    return;
+  }
+  if (NW == 1 || tm.lane < W) {
+    if constexpr (NW == 1) tm.sync(); // every lane has gathered its entries before any writes
+    else __syncwarp();
+#pragma unroll
+    for (int c = 0; c < RPL; c++)
+      if (wl + W * c < NN) b[wl + W * c] = x[c];
+  }
   tm.sync();
 }
 
@@ -534,45 +791,25 @@ struct CellIn {
   double rhoe, rhoesrc;
 };
 
-// The integrator's right-hand side at (t, y) into fy (fKernelSpec).  A free
-// function taking what it reads, so that no caller's state has to live in
-// memory for the call.  Inlined at its call sites by default (drm19 64^3:
-// 909k against 837k cells/s out of line, which keeps one copy of the
-// right-hand side in the kernel; build with -DPPB_RHS_ATTR=__noinline__ for
-// that form).
-#ifndef PPB_RHS_ATTR
-#define PPB_RHS_ATTR __forceinline__
-#endif
 // The right-hand side variants of the integrator (the RHSV template
 // argument): the ideal-gas reactor, the SRK e-reactor, the ideal-gas reactor
 // of a QSS mechanism.  The last two have no analytical Jacobian.
 enum : int { RHS_IDEAL = 0, RHS_SRK = 1, RHS_QSS = 2 };
 
-// The difference-quotient variants (SRK, QSS) evaluate the right-hand
-// side from two call sites, the integrator and the Jacobian's n + 1
-// columns: one out-of-line copy of it (drm19 SRK at 50 atm 39k -> 60k
-// cells/s, CH4_lean_qss 294k -> 672k against the copy inlined at both).
-template <int TEAM, int RHSV>
-__device__ __noinline__ void bdf_rhs_dq(Team<TEAM> tm, const DevMech& M, int rtype, double t, const double* y,
+// The integrator's right-hand side at (t, y) into fy (fKernelSpec), inlined at
+// its one call site (Bdf::drive).  A free function taking what it reads, so
+// that no caller's state has to live in memory for the call.
+template <int TEAM, int RHSV, int NS>
+__device__ __forceinline__ void bdf_rhs(const Team<TEAM>& tm, const DevMech& M, int rtype, double t, const double* y,
                                         double* fy, double rhoe, double rhoesrc, const double* src, double* Y,
-                                        double* sc, double* g, double* qd, double* wdot, double* ei, double* qco)
+                                        double* sc, double* g, double* qd, double* wdot, double* ei, double* qco,
+                                        bool unrounded_e)
 {
   if constexpr (RHSV == RHS_SRK) {
     reactor_rhs_srk<TEAM>(tm, M, t, y, fy, rhoe, rhoesrc, src, Y, sc, g, qd, wdot, ei);
   } else {
-    reactor_rhs<TEAM, RHSV == RHS_QSS>(tm, M, rtype, t, y, fy, rhoe, rhoesrc, src, Y, sc, g, qd, wdot, ei, qco);
-  }
-}
-
-template <int TEAM, int RHSV>
-__device__ PPB_RHS_ATTR void bdf_rhs(Team<TEAM> tm, const DevMech& M, int rtype, double t, const double* y,
-                                     double* fy, double rhoe, double rhoesrc, const double* src, double* Y,
-                                     double* sc, double* g, double* qd, double* wdot, double* ei, double* qco)
-{
-  if constexpr (RHSV == RHS_IDEAL) {
-    reactor_rhs<TEAM, false>(tm, M, rtype, t, y, fy, rhoe, rhoesrc, src, Y, sc, g, qd, wdot, ei, qco);
-  } else {
-    bdf_rhs_dq<TEAM, RHSV>(tm, M, rtype, t, y, fy, rhoe, rhoesrc, src, Y, sc, g, qd, wdot, ei, qco);
+    reactor_rhs<TEAM, RHSV == RHS_QSS, TEAM == 1 ? 0 : NS>(tm, M, rtype, t, y, fy, rhoe, rhoesrc, src, Y, sc, g, qd,
+                                                           wdot, ei, qco, unrounded_e);
   }
 }
 
@@ -584,7 +821,87 @@ struct NoRec {
   static constexpr bool on = false;
 };
 
-template <int NS, int TEAM, typename LT, typename Rec = NoRec, int RHSV = RHS_IDEAL>
+// Cold or shared pieces of the integrator, out of line: one copy of each in a
+// kernel that is bound by instruction fetch (the coefficients of an order, the
+// norm, the power function and the order changes took 15 inlined copies).
+
+// WRMS norm of v[n] with the weights ewt.
+template <int TEAM, int n>
+__device__ __noinline__ double wrms_norm(Team<TEAM> tm, const double* v, const double* ewt)
+{
+  double a = 0.0;
+  for (int i = tm.lane; i < n; i += TEAM) {
+    const double x = v[i] * ewt[i];
+    a += x * x;
+  }
+  return sqrt(tm.sum(a) / n);
+}
+
+// z_j *= eta^j, j = 1..q
+template <int TEAM, int n>
+__device__ __noinline__ void scale_history(Team<TEAM> tm, double* zn, int q, double eta)
+{
+  double factor = eta;
+  for (int j = 1; j <= q; j++) {
+    for (int i = tm.lane; i < n; i += TEAM) zn[j * n + i] *= factor;
+    factor *= eta;
+  }
+  tm.sync();
+}
+
+// The coefficients of order q (cvSetBDF, cvSetTqBDF), by one lane.
+static __device__ __noinline__ void set_bdf_lead(BdfArrays& ar, int q, double h, int qwait)
+{
+  double alpha0, alpha0_hat, xi_inv, xistar_inv, hsum;
+  ar.l[0] = ar.l[1] = xi_inv = xistar_inv = 1.0;
+  for (int i = 2; i <= q; i++) ar.l[i] = 0.0;
+  alpha0 = alpha0_hat = -1.0;
+  hsum = h;
+  if (q > 1) {
+    for (int j = 2; j < q; j++) {
+      hsum += ar.tau[j - 1];
+      xi_inv = h / hsum;
+      alpha0 -= 1.0 / j;
+      for (int i = j; i >= 1; i--) ar.l[i] += ar.l[i - 1] * xi_inv;
+    }
+    alpha0 -= 1.0 / q;
+    xistar_inv = -ar.l[1] - alpha0;
+    hsum += ar.tau[q - 1];
+    xi_inv = h / hsum;
+    alpha0_hat = -ar.l[1] - xi_inv;
+    for (int i = q; i >= 1; i--) ar.l[i] += ar.l[i - 1] * xistar_inv;
+  }
+  const double A1 = 1.0 - alpha0_hat + alpha0;
+  const double A2 = 1.0 + q * A1;
+  ar.tq[2] = fabs(A1 / (alpha0 * A2));
+  ar.tq[5] = fabs(A2 * xistar_inv / (ar.l[q] * xi_inv));
+  if (qwait == 1) {
+    if (q > 1) {
+      const double C = xistar_inv / ar.l[q];
+      const double A3 = alpha0 + 1.0 / q;
+      const double A4 = alpha0_hat + xi_inv;
+      const double Cpinv = (1.0 - A4 + A3) / A3;
+      ar.tq[1] = fabs(C * Cpinv);
+    } else {
+      ar.tq[1] = 1.0;
+    }
+    hsum += ar.tau[q];
+    xi_inv = h / hsum;
+    const double A5 = alpha0 - (1.0 / (q + 1));
+    const double A6 = alpha0_hat - xi_inv;
+    const double Cppinv = (1.0 - A6 + A5) / A2;
+    ar.tq[3] = fabs(Cppinv / (xi_inv * (q + 2) * A5));
+  }
+  ar.tq[4] = 0.1 / ar.tq[2];
+}
+
+// UE: the first residual of a Newton iteration takes the energy of its T solve
+// unrounded (EnergyProduct).  The 16-warp kernels do: on igniting cells one
+// bit of T grows to 1e-8 of the result, so each launch form keeps the rounding
+// its step sequences have always had (with UE false there, LiDryer cells
+// through ignition at rtol = 1e-10 end 9e-9 (2-norm) away; the other launch
+// forms, and every other evaluation, round the energy first).
+template <int NS, int TEAM, typename LT, typename Rec = NoRec, int RHSV = RHS_IDEAL, bool UE = false>
 struct Bdf {
   static constexpr int n = NS + 1;
   static constexpr int PER = (NS + TEAM - 1) / TEAM;
@@ -595,13 +912,16 @@ struct Bdf {
   CellIn cin;
   BdfScalars s;
   BdfArrays& ar;
-  Rec rec;
+  Rec& rec; // an object of its own: its out-of-line calls take its address, not the integrator's
 
-  __device__ Bdf(const Team<TEAM>& t, const DevMech& m, const Options& op, Work<LT>& wk, CellIn ci)
-    : tm(t), M(m), o(op), w(wk), cin(ci), ar(wk.ba[TEAM > 32 ? (t.lane >> 5) : 0])
+  __device__ __forceinline__ Bdf(const Team<TEAM>& t, const DevMech& m, const Options& op, Work<LT>& wk, CellIn ci,
+                                 Rec& rc)
+    : tm(t), M(m), o(op), w(wk), cin(ci), ar(wk.ba[TEAM > 32 ? (t.lane >> 5) : 0]), rec(rc)
   {
   }
 
+  // row j of the Nordsieck array
+  __device__ __forceinline__ double* zn(int j) const { return w.zn + j * n; }
   // the lane that writes this warp's copy of the coefficient arrays
   __device__ __forceinline__ bool lead() const { return (tm.lane % Team<TEAM>::W) == 0; }
   // the warp (or the team's part of it) sees the copy's latest writes
@@ -614,15 +934,7 @@ struct Bdf {
     }
   }
 
-  __device__ __forceinline__ double wrms(const double* v) const
-  {
-    double a = 0.0;
-    for (int i = tm.lane; i < n; i += TEAM) {
-      const double x = v[i] * w.ewt[i];
-      a += x * x;
-    }
-    return sqrt(tm.sum(a) / n);
-  }
+  __device__ __forceinline__ double wrms(const double* v) const { return wrms_norm<TEAM, n>(tm, v, w.ewt); }
 
   __device__ __forceinline__ void set_ewt(const double* y)
   {
@@ -633,29 +945,25 @@ struct Bdf {
     tm.sync();
   }
 
-  // the block rendezvous (when on), then the right-hand side
-  __device__ __forceinline__ void f(double t, const double* y, double* fy)
+  // the right-hand side: the integrator's one call site of it (drive)
+  __device__ __forceinline__ void f(double t, const double* y, double* fy, bool unrounded_e)
   {
-    if (w.rv) rendezvous(w.rv, o.rendezvous);
     PPB_TIC(PH_RHS);
-    bdf_rhs<TEAM, RHSV>(tm, M, o.reactor_type, t, y, fy, cin.rhoe, cin.rhoesrc, w.src, w.Y, w.sc, w.g, w.qd, w.wdot,
-                        w.ei, w.qco);
-    s.nfe++;
+    bdf_rhs<TEAM, RHSV, NS>(tm, M, o.reactor_type, t, y, fy, cin.rhoe, cin.rhoesrc, w.src, w.Y, w.sc, w.g, w.qd, w.wdot,
+                            w.ei, w.qco, unrounded_e);
     PPB_TOC(PH_RHS);
   }
 
+  // the analytical Jacobian (RHS_IDEAL; the other variants' columns are
+  // evaluated by drive)
   __device__ __forceinline__ void jac()
   {
     PPB_TIC(PH_JAC);
-    if constexpr (RHSV != RHS_IDEAL) {
-      jac_dq();
-    } else {
-      // the Newton matrix region is free while the Jacobian is formed: it
-      // holds the per-reaction factors of the warp-cooperative evaluation
-      reactor_jac<TEAM, PER>(tm, M, o.reactor_type, w.y, w.jtmp, w.sc, w.g, w.wdot, w.Y, w.ei, w.h1, w.h2,
-                             TEAM > 1 ? w.qd : nullptr, TEAM > 1 ? w.jx : nullptr);
-      if constexpr (sizeof(LT) != sizeof(double)) jac_to_lt();
-    }
+    // the Newton matrix region is free while the Jacobian is formed: it
+    // holds the per-reaction factors of the warp-cooperative evaluation
+    reactor_jac<TEAM, PER>(tm, M, o.reactor_type, w.y, w.jtmp, w.sc, w.g, w.wdot, w.Y, w.ei, w.h1, w.h2,
+                           TEAM > 1 ? w.qd : nullptr, TEAM > 1 ? w.jx : nullptr);
+    if constexpr (sizeof(LT) != sizeof(double)) jac_to_lt();
     PPB_TOC(PH_JAC);
   }
 
@@ -691,87 +999,40 @@ struct Bdf {
   // CVODE forms it by differences (cvode.solve_type = dense_direct);
   // restated from CVODE's dense difference-quotient Jacobian:
   // column j uses inc = max(sqrt(eps) |y_j|, min_inc / ewt_j), min_inc =
-  // 1000 |h| eps n ||f||_WRMS (1 when ||f|| = 0).  Its RHS evaluations are
-  // not counted in nfe (CVODE counts them separately).
-  __device__ __forceinline__ void jac_dq()
+  // 1000 |h| eps n ||f||_WRMS (1 when ||f|| = 0).  Its RHS evaluations (by
+  // drive, into column j) are not counted in nfe (CVODE counts them
+  // separately).
+  __device__ __forceinline__ double dq_min_inc() const
   {
     const double fnorm = wrms(w.ftemp);
     const double eps = 2.220446049250313e-16;
-    const double srur = sqrt(eps);
-    const double min_inc = (fnorm != 0.0) ? (1000.0 * fabs(s.h) * eps * n * fnorm) : 1.0;
-    for (int i = tm.lane; i < n; i += TEAM) w.tempv[i] = w.y[i];
-    tm.sync();
-    for (int j = 0; j < n; j++) {
-      const double yj = w.tempv[j];
-      const double inc = fmax(srur * fabs(yj), min_inc / w.ewt[j]);
-      tm.sync();
-      if (tm.lane == 0) w.tempv[j] = yj + inc;
-      tm.sync();
-      double* col = w.J + (size_t)j * n;
-      bdf_rhs<TEAM, RHSV>(tm, M, o.reactor_type, s.tn, w.tempv, col, cin.rhoe, cin.rhoesrc, w.src, w.Y, w.sc, w.g,
-                          w.qd, w.wdot, w.ei, w.qco);
-      const double inc_inv = 1.0 / inc;
-      for (int i = tm.lane; i < n; i += TEAM) col[i] = inc_inv * col[i] + (-inc_inv) * w.ftemp[i];
-      if (tm.lane == 0) w.tempv[j] = yj;
-      tm.sync();
-    }
+    return (fnorm != 0.0) ? (1000.0 * fabs(s.h) * eps * n * fnorm) : 1.0;
   }
 
-  __device__ __forceinline__ int hin(double tout)
+  // perturb component j of tempv (a copy of y); returns the increment
+  __device__ __forceinline__ double dq_perturb(int j, double min_inc)
   {
-    const double tdiff = tout - s.tn;
-    if (tdiff == 0.0) return ST_TOO_CLOSE;
-    const double tdist = fabs(tdiff);
-    const double tround = 2.220446049250313e-16 * fmax(fabs(s.tn), fabs(tout));
-    if (tdist < 2.0 * tround) return ST_TOO_CLOSE;
-    const double hlb = 100.0 * tround;
-    double hub_inv = 0.0;
-    for (int i = tm.lane; i < n; i += TEAM) {
-      const double t1 = 0.1 * fabs(w.zn[0][i]) + 1.0 / w.ewt[i];
-      hub_inv = fmax(hub_inv, fabs(w.zn[1][i]) / t1);
-    }
-    hub_inv = tm.max(hub_inv);
-    double hub = 0.1 * tdist;
-    if (hub * hub_inv > 1.0) hub = 1.0 / hub_inv;
-    double hg = sqrt(hlb * hub);
-    if (hub < hlb) {
-      s.h = hg;
-      return ST_OK;
-    }
-    double hnew = hg;
-    for (int count1 = 1; count1 <= 4; count1++) {
-      for (int i = tm.lane; i < n; i += TEAM) w.y[i] = hg * w.zn[1][i] + w.zn[0][i];
-      tm.sync();
-      f(s.tn + hg, w.y, w.tempv);
-      for (int i = tm.lane; i < n; i += TEAM) w.tempv[i] = (w.tempv[i] - w.zn[1][i]) * (1.0 / hg);
-      tm.sync();
-      const double yddnrm = wrms(w.tempv);
-      hnew = (yddnrm * hub * hub > 2.0) ? sqrt(2.0 / yddnrm) : sqrt(hg * hub);
-      if (count1 == 4) break;
-      const double hrat = hnew / hg;
-      if (hrat > 0.5 && hrat < 2.0) break;
-      if (count1 > 1 && hrat > 2.0) {
-        hnew = hg;
-        break;
-      }
-      hg = hnew;
-    }
-    double h0 = 0.5 * hnew;
-    if (h0 < hlb) h0 = hlb;
-    if (h0 > hub) h0 = hub;
-    s.h = h0;
-    return ST_OK;
+    const double yj = w.y[j];
+    const double inc = fmax(sqrt(2.220446049250313e-16) * fabs(yj), min_inc / w.ewt[j]);
+    if (tm.lane == 0) w.tempv[j] = yj + inc;
+    tm.sync();
+    return inc;
+  }
+
+  // column j from the right-hand side at the perturbed state
+  __device__ __forceinline__ void dq_column(int j, double inc)
+  {
+    double* col = w.jtmp + (size_t)j * n;
+    const double inc_inv = 1.0 / inc;
+    for (int i = tm.lane; i < n; i += TEAM) col[i] = inc_inv * col[i] + (-inc_inv) * w.ftemp[i];
+    if (tm.lane == 0) w.tempv[j] = w.y[j];
+    tm.sync();
   }
 
   __device__ __forceinline__ void rescale()
   {
     if constexpr (Rec::on) rec.rescale(tm, s.q, s.eta);
-    double factor = s.eta;
-    for (int j = 1; j <= s.q; j++) {
-      for (int i = tm.lane; i < n; i += TEAM) w.zn[j][i] *= factor;
-      factor *= s.eta;
-    }
-    tm.sync();
+    scale_history<TEAM, n>(tm, w.zn, s.q, s.eta);
     s.h = s.hscale * s.eta;
     s.hscale = s.h;
   }
@@ -781,7 +1042,7 @@ struct Bdf {
     s.tn += s.h;
     for (int i = tm.lane; i < n; i += TEAM) {
       for (int k = 1; k <= s.q; k++)
-        for (int j = s.q; j >= k; j--) w.zn[j - 1][i] += w.zn[j][i];
+        for (int j = s.q; j >= k; j--) zn(j - 1)[i] += zn(j)[i];
     }
     tm.sync();
   }
@@ -791,7 +1052,7 @@ struct Bdf {
     s.tn = saved_t;
     for (int i = tm.lane; i < n; i += TEAM) {
       for (int k = 1; k <= s.q; k++)
-        for (int j = s.q; j >= k; j--) w.zn[j - 1][i] -= w.zn[j][i];
+        for (int j = s.q; j >= k; j--) zn(j - 1)[i] -= zn(j)[i];
     }
     tm.sync();
   }
@@ -799,56 +1060,9 @@ struct Bdf {
   // the coefficients of order q: written by the lead lane only
   __device__ __forceinline__ void set_bdf()
   {
-    if (lead()) set_bdf_lead();
+    if (lead()) set_bdf_lead(ar, s.q, s.h, s.qwait);
     wsync();
   }
-
-  __device__ __forceinline__ void set_bdf_lead()
-  {
-    double alpha0, alpha0_hat, xi_inv, xistar_inv, hsum;
-    const int q = s.q;
-    ar.l[0] = ar.l[1] = xi_inv = xistar_inv = 1.0;
-    for (int i = 2; i <= q; i++) ar.l[i] = 0.0;
-    alpha0 = alpha0_hat = -1.0;
-    hsum = s.h;
-    if (q > 1) {
-      for (int j = 2; j < q; j++) {
-        hsum += ar.tau[j - 1];
-        xi_inv = s.h / hsum;
-        alpha0 -= 1.0 / j;
-        for (int i = j; i >= 1; i--) ar.l[i] += ar.l[i - 1] * xi_inv;
-      }
-      alpha0 -= 1.0 / q;
-      xistar_inv = -ar.l[1] - alpha0;
-      hsum += ar.tau[q - 1];
-      xi_inv = s.h / hsum;
-      alpha0_hat = -ar.l[1] - xi_inv;
-      for (int i = q; i >= 1; i--) ar.l[i] += ar.l[i - 1] * xistar_inv;
-    }
-    const double A1 = 1.0 - alpha0_hat + alpha0;
-    const double A2 = 1.0 + q * A1;
-    ar.tq[2] = fabs(A1 / (alpha0 * A2));
-    ar.tq[5] = fabs(A2 * xistar_inv / (ar.l[q] * xi_inv));
-    if (s.qwait == 1) {
-      if (q > 1) {
-        const double C = xistar_inv / ar.l[q];
-        const double A3 = alpha0 + 1.0 / q;
-        const double A4 = alpha0_hat + xi_inv;
-        const double Cpinv = (1.0 - A4 + A3) / A3;
-        ar.tq[1] = fabs(C * Cpinv);
-      } else {
-        ar.tq[1] = 1.0;
-      }
-      hsum += ar.tau[q];
-      xi_inv = s.h / hsum;
-      const double A5 = alpha0 - (1.0 / (q + 1));
-      const double A6 = alpha0_hat - xi_inv;
-      const double Cppinv = (1.0 - A6 + A5) / A2;
-      ar.tq[3] = fabs(Cppinv / (xi_inv * (q + 2) * A5));
-    }
-    ar.tq[4] = 0.1 / ar.tq[2];
-  }
-
   __device__ __forceinline__ void set()
   {
     set_bdf();
@@ -858,28 +1072,17 @@ struct Bdf {
     s.gamrat = (s.nst > 0) ? s.gamma / s.gammap : 1.0;
   }
 
-  // cvLsSetup: (re)use J, form I - gamma J, factor
-  __device__ __forceinline__ int ls_setup(int convfail)
+  // whether the setup needs a new Jacobian (cvLsSetup)
+  __device__ __forceinline__ bool need_jac(int convfail) const
   {
     const double dgamma = fabs((s.gamma / s.gammap) - 1.0);
-    const bool jbad = (s.nst == 0) || (s.nst >= s.nstlj + o.jac_eval_freq) || ((convfail == 1) && (dgamma < 0.2)) ||
-                      (convfail == 2);
-    if (!jbad) {
-      s.jcur = 0;
-    } else {
-      if (lead()) ar.nje++;
-      s.nstlj = s.nst;
-      s.jcur = 1;
-      // the Jacobian is the longest stretch a team runs alone (drm19: ~300k
-      // SM clocks, against ~34k for a right-hand side and ~65k for a
-      // factorisation): the team leaves the block rendezvous meanwhile, so
-      // that the other teams' right-hand sides do not wait for it (drm19
-      // 64^3: 1.047M cells/s against 0.96M; leaving it for the
-      // factorisations too gave 0.55M, as the teams then drift apart)
-      rendezvous_leave(w.rv);
-      jac();
-      rendezvous_resume(w.rv);
-    }
+    return (s.nst == 0) || (s.nst >= s.nstlj + o.jac_eval_freq) || ((convfail == 1) && (dgamma < 0.2)) ||
+           (convfail == 2);
+  }
+
+  // form I - gamma J and factor it
+  __device__ __forceinline__ int ls_factor()
+  {
     s.gamma_lu = s.gamma;
     PPB_TIC(PH_LU);
     for (int i = tm.lane; i < n; i += TEAM) {
@@ -890,9 +1093,12 @@ struct Bdf {
       }
     }
     tm.sync();
-    const int ier = lu_factor<TEAM, LT>(tm, w.A, n, w.piv) ? 1 : 0;
-    if constexpr ((TEAM == 16 || TEAM == 32) && n <= TEAM) {
-      if (!ier) perm_from_piv(tm, w.piv, w.perm, n);
+    int ier;
+    if constexpr (TEAM > 1) {
+      ier = lu_factor_team<TEAM, LT, (n + Team<TEAM>::W - 1) / Team<TEAM>::W>(tm, w.A, n, w.piv, w.perm) ? 1 : 0;
+      if (!ier) diag_recip(tm, w.A, w.dinv, n);
+    } else {
+      ier = lu_factor<LT>(w.A, n, w.piv) ? 1 : 0;
     }
     PPB_TOC(PH_LU);
     return ier;
@@ -901,8 +1107,8 @@ struct Bdf {
   // (LU) x = b in place with the current factor
   __device__ __forceinline__ void lsolve(double* b)
   {
-    if constexpr ((TEAM == 16 || TEAM == 32) && n <= TEAM) {
-      lu_solve_reg<TEAM, LT, n>(tm, w.A, w.perm, b);
+    if constexpr (TEAM > 1) {
+      lu_solve_reg<TEAM, LT, n>(tm, w.A, w.piv, w.perm, w.dinv, b);
     } else {
       lu_solve<TEAM, LT>(tm, w.A, n, w.piv, b);
     }
@@ -945,90 +1151,6 @@ struct Bdf {
     }
   }
 
-  __device__ __forceinline__ void nls_residual()
-  {
-    for (int i = tm.lane; i < n; i += TEAM) w.y[i] = w.zn[0][i] + w.acor[i];
-    tm.sync();
-    f(s.tn, w.y, w.ftemp);
-    for (int i = tm.lane; i < n; i += TEAM) {
-      const double r = s.rl1 * w.zn[1][i] + w.acor[i];
-      w.delta[i] = -s.gamma * w.ftemp[i] + r;
-    }
-    tm.sync();
-  }
-
-  __device__ __forceinline__ int nls(int nflag)
-  {
-    PPB_TIC(PH_NEWTON);
-    const int r = nls_impl(nflag);
-    PPB_TOC(PH_NEWTON);
-    return r;
-  }
-
-  __device__ __forceinline__ int nls_impl(int nflag)
-  {
-    const int convfail = ((nflag == 0) || (nflag == 2)) ? 0 : 2;
-    bool callSetup = (nflag == 1) || (nflag == 2) || (s.nst == 0) || (s.nst >= s.nstlp + 20) ||
-                     (fabs(s.gamrat - 1.0) > 0.3);
-    for (int i = tm.lane; i < n; i += TEAM) w.acor[i] = 0.0;
-    tm.sync();
-    bool jbad = false;
-    int retval = 0;
-    for (;;) {
-      nls_residual();
-      if (callSetup) {
-        const int ier = ls_setup(jbad ? 1 : convfail);
-        if (lead()) ar.nsetups++;
-        s.gamrat = 1.0;
-        s.gammap = s.gamma;
-        s.crate = 1.0;
-        s.nstlp = s.nst;
-        if (ier) return -1;
-      }
-      int m = 0;
-      for (;;) {
-        if (lead()) ar.nni++;
-        for (int i = tm.lane; i < n; i += TEAM) w.delta[i] = -w.delta[i];
-        tm.sync();
-        ls_solve();
-        if (s.gamrat != 1.0) {
-          const double sc = 2.0 / (1.0 + s.gamrat);
-          for (int i = tm.lane; i < n; i += TEAM) w.delta[i] *= sc;
-        }
-        for (int i = tm.lane; i < n; i += TEAM) w.acor[i] += w.delta[i];
-        tm.sync();
-        const double del = wrms(w.delta);
-        if (m > 0) s.crate = fmax(0.3 * s.crate, del / s.delp);
-        const double dcon = del * fmin(1.0, s.crate) / ar.tq[4];
-        if (dcon <= 1.0) {
-          s.acnrm = (m == 0) ? del : wrms(w.acor);
-          s.jcur = 0;
-          return 0;
-        }
-        if ((m >= 1) && (del > 2.0 * s.delp)) {
-          retval = 1;
-          break;
-        }
-        s.delp = del;
-        m++;
-        if (m >= o.max_nls_iters) {
-          retval = 1;
-          break;
-        }
-        nls_residual();
-      }
-      if (retval > 0 && !s.jcur) {
-        callSetup = true;
-        jbad = true;
-        for (int i = tm.lane; i < n; i += TEAM) w.acor[i] = 0.0;
-        tm.sync();
-        continue;
-      }
-      break;
-    }
-    return retval;
-  }
-
   __device__ __forceinline__ void increase_bdf()
   {
     double alpha0, alpha1, prod, xi, xiold, hsum, A1;
@@ -1055,9 +1177,9 @@ struct Bdf {
     wsync();
     A1 = (-alpha0 - alpha1) / prod;
     for (int i = tm.lane; i < n; i += TEAM) {
-      const double zL = A1 * w.zn[s.indx_acor][i];
-      w.zn[s.L][i] = zL;
-      for (int j = 2; j <= s.q; j++) w.zn[j][i] += ar.l[j] * zL;
+      const double zL = A1 * zn(s.indx_acor)[i];
+      zn(s.L)[i] = zL;
+      for (int j = 2; j <= s.q; j++) zn(j)[i] += ar.l[j] * zL;
     }
     tm.sync();
     if constexpr (Rec::on) rec.increase(tm, s.q, s.L, s.indx_acor, A1, ar.l);
@@ -1077,7 +1199,7 @@ struct Bdf {
     }
     wsync();
     for (int i = tm.lane; i < n; i += TEAM)
-      for (int j = 2; j < s.q; j++) w.zn[j][i] -= ar.l[j] * w.zn[s.q][i];
+      for (int j = 2; j < s.q; j++) zn(j)[i] -= ar.l[j] * zn(s.q)[i];
     tm.sync();
     if constexpr (Rec::on) rec.decrease(tm, s.q, ar.l);
   }
@@ -1115,7 +1237,7 @@ struct Bdf {
     if (nef == o.max_err_fails) return ST_ERR_FAILURE;
     s.etamax = 1.0;
     if (nef <= 3) {
-      s.eta = 1.0 / (pow(6.0 * dsm, 1.0 / s.L) + 1.0e-6);
+      s.eta = 1.0 / (ppb_pow(6.0 * dsm, 1.0 / s.L) + 1.0e-6);
       s.eta = fmax(0.1, s.eta);
       if (nef >= 2) s.eta = fmin(s.eta, 0.2);
       rescale();
@@ -1134,11 +1256,7 @@ struct Bdf {
     s.h *= s.eta;
     s.hscale = s.h;
     s.qwait = 10;
-    f(s.tn, w.zn[0], w.tempv);
-    for (int i = tm.lane; i < n; i += TEAM) w.zn[1][i] = s.h * w.tempv[i];
-    tm.sync();
-    if constexpr (Rec::on) rec.freset(tm, s.tn, s.h, w.zn[0]);
-    return 5;
+    return 6; // restart the history from f(tn, zn_0)
   }
 
   __device__ __forceinline__ void complete_step()
@@ -1155,12 +1273,12 @@ struct Bdf {
     wsync();
     if constexpr (Rec::on) {
       rec.predict(tm, s.q);
-      rec.correct(tm, s.q, save, s.tn, s.gamma, s.rl1, ar.l, w.zn[0], w.acor);
+      rec.correct(tm, s.q, save, s.tn, s.gamma, s.rl1, ar.l, zn(0), w.acor);
     }
     for (int i = tm.lane; i < n; i += TEAM) {
       const double a = w.acor[i];
-      for (int j = 0; j <= s.q; j++) w.zn[j][i] += ar.l[j] * a;
-      if (save) w.zn[s.qmax][i] = a;
+      for (int j = 0; j <= s.q; j++) zn(j)[i] += ar.l[j] * a;
+      if (save) zn(s.qmax)[i] = a;
     }
     tm.sync();
     s.qwait--;
@@ -1187,7 +1305,7 @@ struct Bdf {
       s.eta = 1.0;
       return;
     }
-    const double etaq = 1.0 / (pow(6.0 * dsm, 1.0 / s.L) + 1.0e-6);
+    const double etaq = 1.0 / (ppb_pow(6.0 * dsm, 1.0 / s.L) + 1.0e-6);
     if (s.qwait != 0) {
       s.eta = etaq;
       s.qprime = s.q;
@@ -1197,16 +1315,16 @@ struct Bdf {
     s.qwait = 2;
     double etaqm1 = 0.0;
     if (s.q > 1) {
-      const double ddn = wrms(w.zn[s.q]) * ar.tq[1];
-      etaqm1 = 1.0 / (pow(6.0 * ddn, 1.0 / s.q) + 1.0e-6);
+      const double ddn = wrms(zn(s.q)) * ar.tq[1];
+      etaqm1 = 1.0 / (ppb_pow(6.0 * ddn, 1.0 / s.q) + 1.0e-6);
     }
     double etaqp1 = 0.0;
     if (s.q != s.qmax && ar.saved_tq5 != 0.0) {
-      const double cquot = (ar.tq[5] / ar.saved_tq5) * pow(s.h / ar.tau[2], (double)s.L);
-      for (int i = tm.lane; i < n; i += TEAM) w.tempv[i] = -cquot * w.zn[s.qmax][i] + w.acor[i];
+      const double cquot = (ar.tq[5] / ar.saved_tq5) * ppb_pow(s.h / ar.tau[2], (double)s.L);
+      for (int i = tm.lane; i < n; i += TEAM) w.tempv[i] = -cquot * zn(s.qmax)[i] + w.acor[i];
       tm.sync();
       const double dup = wrms(w.tempv) * ar.tq[3];
-      etaqp1 = 1.0 / (pow(10.0 * dup, 1.0 / (s.L + 1)) + 1.0e-6);
+      etaqp1 = 1.0 / (ppb_pow(10.0 * dup, 1.0 / (s.L + 1)) + 1.0e-6);
     }
     const double etam = fmax(etaqm1, fmax(etaq, etaqp1));
     if ((etam > 0.0) && (etam < 1.5)) {
@@ -1221,7 +1339,7 @@ struct Bdf {
     } else {
       s.eta = etaqp1;
       s.qprime = s.q + 1;
-      for (int i = tm.lane; i < n; i += TEAM) w.zn[s.qmax][i] = w.acor[i];
+      for (int i = tm.lane; i < n; i += TEAM) zn(s.qmax)[i] = w.acor[i];
       tm.sync();
       if constexpr (Rec::on) rec.saveqmax(tm);
     }
@@ -1239,87 +1357,318 @@ struct Bdf {
     rescale();
   }
 
-  __device__ __forceinline__ int step()
-  {
-    PPB_TIC(PH_STEP);
-    const int r = step_impl();
-    PPB_TOC(PH_STEP);
-    return r;
-  }
+  // The integration as one loop around one evaluation of the right-hand
+  // side.  Every step of the algorithm that needs f sets the evaluation's
+  // time, input and output and the phase that takes its result; so the kernel
+  // holds one copy of the right-hand side (and of the Newton iteration, the
+  // factorisation and the solve), and warps that meet at the rendezvous run
+  // the same instructions whatever they need f for.  With a copy at each of
+  // the integrator's five call sites, the 16-warp drm19 kernel ran 520k cells/s
+  // (64^3 field) against 890k with them shared: its warps fetched different
+  // copies.
+  enum : int { EV_START, EV_HIN, EV_NEWTON_FIRST, EV_NEWTON, EV_RESET, EV_JCOL };
 
-  __device__ __forceinline__ int step_impl()
-  {
-    const double saved_t = s.tn;
-    int ncf = 0, nef = 0, nflag = 0;
-    double dsm = 0.0;
-    if ((s.nst > 0) && (s.hprime != s.h)) adjust_params();
-    for (;;) {
-      predict();
-      set();
-      nflag = nls(nflag);
-      const int kflag = handle_nflag(nflag, saved_t, ncf);
-      if (kflag == 3) continue;
-      if (kflag != 2) return kflag;
-      const int eflag = do_error_test(nflag, saved_t, nef, dsm);
-      if (eflag == 5) continue;
-      if (eflag != ST_OK) return eflag;
-      break;
-    }
-    complete_step();
-    prepare_next_step(dsm);
-    s.etamax = 10.0;
-    return ST_OK;
-  }
-
-  // Start of an integration of w.zn[0] (initial y, team-shared) towards
-  // tout: history, error weights, initial step (cvInitialSetup, cvHin).
-  __device__ __forceinline__ int start(double tout)
-  {
-    s = BdfScalars{};
-    if (lead()) ar = BdfArrays{};
-    // no factorisation yet: identity pivots and row order (a checkpoint taken
-    // before the first step holds valid ones)
-    for (int i = tm.lane; i < n; i += TEAM) {
-      w.piv[i] = i;
-      w.perm[i] = i;
-    }
-    tm.sync();
-    s.qmax = o.max_order;
-    s.q = 1;
-    s.L = 2;
-    s.qwait = 2;
-    s.etamax = 10000.0;
-    s.tn = 0.0;
-    set_ewt(w.zn[0]);
-    f(s.tn, w.zn[0], w.zn[1]);
-    const int flag = hin(tout);
-    if (flag == ST_OK) {
-      s.hscale = s.h;
-      s.hprime = s.h;
-      for (int i = tm.lane; i < n; i += TEAM) w.zn[1][i] *= s.h;
-      tm.sync();
-      if constexpr (Rec::on) rec.init(tm, s.h, w.zn[0]);
-    }
-    return flag;
-  }
-
-  // Step until tout is passed (then interpolate to tout into w.y and set
-  // done) or, with a recorder, until the recorder closes its segment.
-  // nstloc counts the steps of this call to react.
-  __device__ __forceinline__ int advance(double tout, int& nstloc, bool& done)
+  // fresh: integrate from w.zn (initial y, team-shared) towards tout --
+  // history, error weights, initial step (cvInitialSetup, cvHin); with a
+  // recorder it returns when that is done.  Otherwise step on until tout is
+  // passed (then interpolate to tout into w.y and set done) or, with a
+  // recorder, until the recorder closes its segment.  nstloc counts the
+  // steps of this call to react.
+  __device__ __forceinline__ int drive(double tout, int& nstloc, bool& done, bool fresh)
   {
     done = false;
+    double ft;         // the evaluation: time,
+    const double* fin; // state,
+    double* fout;      // result,
+    int ev;            // and what takes it
+    // initial step
+    double hlb = 0.0, hub = 0.0, hg = 0.0;
+    int count1 = 0;
+    // the step
+    double saved_t = 0.0;
+    int ncf = 0, nef = 0, nflag = 0;
+    // the Newton iteration
+    int convfail = 0, m = 0;
+    bool callSetup = false;
+    // the difference-quotient Jacobian's column
+    int jcol = 0;
+    double dq_min = 0.0, dq_inc = 0.0;
+
+    enum : int { GO_STEP, GO_PREDICT, GO_RESIDUAL, GO_EVAL };
+    int go;
+    if (fresh) {
+      s = BdfScalars{};
+      if (lead()) ar = BdfArrays{};
+      // no factorisation yet: identity pivots and row order (a checkpoint taken
+      // before the first step holds valid ones)
+      for (int i = tm.lane; i < n; i += TEAM) {
+        w.piv[i] = i;
+        w.perm[i] = i;
+      }
+      tm.sync();
+      s.qmax = o.max_order;
+      s.q = 1;
+      s.L = 2;
+      s.qwait = 2;
+      s.etamax = 10000.0;
+      s.tn = 0.0;
+      set_ewt(zn(0));
+      ft = s.tn;
+      fin = zn(0);
+      fout = zn(1);
+      ev = EV_START;
+      go = GO_EVAL;
+    } else {
+      ft = 0.0;
+      fin = w.y;
+      fout = w.ftemp;
+      ev = EV_NEWTON_FIRST;
+      go = GO_STEP;
+    }
     for (;;) {
-      if (s.nst > 0) set_ewt(w.zn[0]);
-      if (nstloc >= o.max_steps) return ST_TOO_MUCH_WORK;
-      const int flag = step();
-      if (flag != ST_OK) return flag;
+      if (go == GO_STEP) {
+        if (s.nst > 0) set_ewt(zn(0));
+        if (nstloc >= o.max_steps) return ST_TOO_MUCH_WORK;
+        saved_t = s.tn;
+        ncf = nef = nflag = 0;
+        if ((s.nst > 0) && (s.hprime != s.h)) adjust_params();
+        go = GO_PREDICT;
+      }
+      if (go == GO_PREDICT) {
+        predict();
+        set();
+        convfail = ((nflag == 0) || (nflag == 2)) ? 0 : 2;
+        callSetup = (nflag == 1) || (nflag == 2) || (s.nst == 0) || (s.nst >= s.nstlp + 20) ||
+                    (fabs(s.gamrat - 1.0) > 0.3);
+        for (int i = tm.lane; i < n; i += TEAM) w.acor[i] = 0.0;
+        tm.sync();
+        ev = EV_NEWTON_FIRST;
+        go = GO_RESIDUAL;
+      }
+      if (go == GO_RESIDUAL) {
+        for (int i = tm.lane; i < n; i += TEAM) w.y[i] = zn(0)[i] + w.acor[i];
+        tm.sync();
+        ft = s.tn;
+        fin = w.y;
+        fout = w.ftemp;
+      }
+      // ---- the evaluation (the block rendezvous before it, when on; a
+      // difference-quotient Jacobian is formed outside it)
+      if (w.rv && ev != EV_JCOL) rendezvous(w.rv, o.rendezvous);
+      f(ft, fin, fout, UE && ev == EV_NEWTON_FIRST);
+      if (RHSV == RHS_IDEAL || ev != EV_JCOL) s.nfe++;
+
+      // ---- what takes its result
+      if (ev == EV_START || ev == EV_HIN) {
+        int flag = ST_OK;
+        bool more = false; // another evaluation of the initial-step estimate
+        double hnew = hg;
+        if (ev == EV_START) {
+          const double tdiff = tout - s.tn;
+          const double tdist = fabs(tdiff);
+          const double tround = 2.220446049250313e-16 * fmax(fabs(s.tn), fabs(tout));
+          if (tdiff == 0.0 || tdist < 2.0 * tround) return ST_TOO_CLOSE;
+          hlb = 100.0 * tround;
+          double hub_inv = 0.0;
+          for (int i = tm.lane; i < n; i += TEAM) {
+            const double t1 = 0.1 * fabs(zn(0)[i]) + 1.0 / w.ewt[i];
+            hub_inv = fmax(hub_inv, fabs(zn(1)[i]) / t1);
+          }
+          hub_inv = tm.max(hub_inv);
+          hub = 0.1 * tdist;
+          if (hub * hub_inv > 1.0) hub = 1.0 / hub_inv;
+          hg = sqrt(hlb * hub);
+          count1 = 1;
+          if (hub < hlb) {
+            s.h = hg;
+          } else {
+            more = true;
+          }
+        } else {
+          for (int i = tm.lane; i < n; i += TEAM) w.tempv[i] = (w.tempv[i] - zn(1)[i]) * (1.0 / hg);
+          tm.sync();
+          const double yddnrm = wrms(w.tempv);
+          hnew = (yddnrm * hub * hub > 2.0) ? sqrt(2.0 / yddnrm) : sqrt(hg * hub);
+          const double hrat = hnew / hg;
+          more = !(count1 == 4 || (hrat > 0.5 && hrat < 2.0));
+          if (more && count1 > 1 && hrat > 2.0) {
+            hnew = hg;
+            more = false;
+          }
+          if (more) {
+            hg = hnew;
+            count1++;
+          } else {
+            double h0 = 0.5 * hnew;
+            if (h0 < hlb) h0 = hlb;
+            if (h0 > hub) h0 = hub;
+            s.h = h0;
+          }
+        }
+        if (more) {
+          for (int i = tm.lane; i < n; i += TEAM) w.y[i] = hg * zn(1)[i] + zn(0)[i];
+          tm.sync();
+          ft = s.tn + hg;
+          fin = w.y;
+          fout = w.tempv;
+          ev = EV_HIN;
+          go = GO_EVAL;
+          continue;
+        }
+        s.hscale = s.h;
+        s.hprime = s.h;
+        for (int i = tm.lane; i < n; i += TEAM) zn(1)[i] *= s.h;
+        tm.sync();
+        if constexpr (Rec::on) {
+          rec.init(tm, s.h, zn(0));
+          return flag;
+        }
+        go = GO_STEP;
+        continue;
+      }
+      if (ev == EV_RESET) {
+        for (int i = tm.lane; i < n; i += TEAM) zn(1)[i] = s.h * w.tempv[i];
+        tm.sync();
+        if constexpr (Rec::on) rec.freset(tm, s.tn, s.h, zn(0));
+        go = GO_PREDICT;
+        continue;
+      }
+      bool factor = false;
+      if (RHSV != RHS_IDEAL && ev == EV_JCOL) {
+        dq_column(jcol, dq_inc);
+        if (++jcol < n) {
+          dq_inc = dq_perturb(jcol, dq_min);
+          fout = w.jtmp + (size_t)jcol * n;
+          continue;
+        }
+        rendezvous_resume(w.rv);
+        factor = true;
+      } else {
+        // the residual of the nonlinear system
+        for (int i = tm.lane; i < n; i += TEAM) {
+          const double r = s.rl1 * zn(1)[i] + w.acor[i];
+          w.delta[i] = -s.gamma * w.ftemp[i] + r;
+        }
+        tm.sync();
+        if (ev == EV_NEWTON_FIRST) {
+          m = 0;
+          if (callSetup) {
+            if (need_jac(convfail)) {
+              if (lead()) ar.nje++;
+              s.nstlj = s.nst;
+              s.jcur = 1;
+              // the Jacobian is the longest stretch a team runs alone: the
+              // team leaves the block rendezvous meanwhile, so that the other
+              // teams' right-hand sides do not wait for it (drm19 64^3: 1.047M
+              // cells/s against 0.96M; leaving it for the factorisations too
+              // gave 0.55M, as the teams then drift apart)
+              rendezvous_leave(w.rv);
+              if constexpr (RHSV != RHS_IDEAL) {
+                dq_min = dq_min_inc();
+                for (int i = tm.lane; i < n; i += TEAM) w.tempv[i] = w.y[i];
+                tm.sync();
+                jcol = 0;
+                dq_inc = dq_perturb(0, dq_min);
+                ft = s.tn;
+                fin = w.tempv;
+                fout = w.jtmp;
+                ev = EV_JCOL;
+                go = GO_EVAL;
+                continue;
+              } else {
+                jac();
+                rendezvous_resume(w.rv);
+              }
+            } else {
+              s.jcur = 0;
+            }
+            factor = true;
+          }
+        }
+      }
+      int ier = 0;
+      if (factor) {
+        ier = ls_factor();
+        if (lead()) ar.nsetups++;
+        s.gamrat = 1.0;
+        s.gammap = s.gamma;
+        s.crate = 1.0;
+        s.nstlp = s.nst;
+      }
+      // one Newton iteration; r: -1 the setup failed, 0 converged, 1 not, 2 go on
+      int r = -1;
+      if (!ier) {
+        if (lead()) ar.nni++;
+        for (int i = tm.lane; i < n; i += TEAM) w.delta[i] = -w.delta[i];
+        tm.sync();
+        ls_solve();
+        if (s.gamrat != 1.0) {
+          const double sc = 2.0 / (1.0 + s.gamrat);
+          for (int i = tm.lane; i < n; i += TEAM) w.delta[i] *= sc;
+        }
+        for (int i = tm.lane; i < n; i += TEAM) w.acor[i] += w.delta[i];
+        tm.sync();
+        const double del = wrms(w.delta);
+        if (m > 0) s.crate = fmax(0.3 * s.crate, del / s.delp);
+        const double dcon = del * fmin(1.0, s.crate) / ar.tq[4];
+        if (dcon <= 1.0) {
+          s.acnrm = (m == 0) ? del : wrms(w.acor);
+          s.jcur = 0;
+          r = 0;
+        } else if ((m >= 1) && (del > 2.0 * s.delp)) {
+          r = 1;
+        } else {
+          s.delp = del;
+          m++;
+          r = (m >= o.max_nls_iters) ? 1 : 2;
+        }
+        if (r == 2) {
+          ev = EV_NEWTON;
+          go = GO_RESIDUAL;
+          continue;
+        }
+        if (r == 1 && !s.jcur) {
+          // again from the predictor with a fresh Jacobian
+          callSetup = true;
+          convfail = 1;
+          for (int i = tm.lane; i < n; i += TEAM) w.acor[i] = 0.0;
+          tm.sync();
+          ev = EV_NEWTON_FIRST;
+          go = GO_RESIDUAL;
+          continue;
+        }
+      }
+      nflag = r;
+      const int kflag = handle_nflag(nflag, saved_t, ncf);
+      if (kflag == 3) {
+        go = GO_PREDICT;
+        continue;
+      }
+      if (kflag != 2) return kflag;
+      double dsm = 0.0;
+      const int eflag = do_error_test(nflag, saved_t, nef, dsm);
+      if (eflag == 5) {
+        go = GO_PREDICT;
+        continue;
+      }
+      if (eflag == 6) {
+        ft = s.tn;
+        fin = zn(0);
+        fout = w.tempv;
+        ev = EV_RESET;
+        go = GO_EVAL;
+        continue;
+      }
+      if (eflag != ST_OK) return eflag;
+      complete_step();
+      prepare_next_step(dsm);
+      s.etamax = 10.0;
       nstloc++;
       if ((s.tn - tout) * s.h >= 0.0) {
         const double sfac = (tout - s.tn) / s.h;
         for (int i = tm.lane; i < n; i += TEAM) {
-          double v = w.zn[s.q][i];
-          for (int j = s.q - 1; j >= 0; j--) v = w.zn[j][i] + sfac * v;
+          double v = zn(s.q)[i];
+          for (int j = s.q - 1; j >= 0; j--) v = zn(j)[i] + sfac * v;
           w.y[i] = v;
         }
         tm.sync();
@@ -1330,21 +1679,19 @@ struct Bdf {
       if constexpr (Rec::on) {
         if (rec.segment_full()) return ST_OK;
       }
+      go = GO_STEP;
     }
   }
 
-  // Integrate w.zn[0] (initial y, team-shared) over [0, tout]; result in w.y.
+  // Integrate w.zn (initial y, team-shared) over [0, tout]; result in w.y.
   __device__ __forceinline__ int run(double tout)
   {
     PPB_TIC(PH_TOTAL);
-    int flag = start(tout);
-    if (flag == ST_OK) {
-      int nstloc = 0;
-      bool done = false;
-      flag = advance(tout, nstloc, done);
-    }
+    int nstloc = 0;
+    bool done = false;
+    const int flag = drive(tout, nstloc, done, true);
     if (flag != ST_OK) {
-      for (int i = tm.lane; i < n; i += TEAM) w.y[i] = w.zn[0][i];
+      for (int i = tm.lane; i < n; i += TEAM) w.y[i] = zn(0)[i];
       tm.sync();
     }
     PPB_TOC(PH_TOTAL);
@@ -1358,7 +1705,7 @@ struct Bdf {
 
 // ReactorRK64.cpp:73-144 for one cell (team).  y (team-shared) in/out;
 // returns the number of RK steps.
-template <int TEAM, typename LT>
+template <int NS, int TEAM, typename LT>
 __device__ int rk64_cell(const Team<TEAM>& tm, const DevMech& M, const Options& o, Work<LT>& w, CellIn cin,
                          double dt)
 {
@@ -1370,8 +1717,8 @@ __device__ int rk64_cell(const Team<TEAM>& tm, const DevMech& M, const Options& 
                          -0.219084567203338, 0.164022338959433, 0.0426421977505659};
   const int neq = M.nsp + 1;
   double* soln = w.y;
-  double* carry = w.zn[0];
-  double* error = w.zn[1];
+  double* carry = w.zn;
+  double* error = w.zn + neq;
   double* ydot = w.ftemp;
   for (int i = tm.lane; i < neq; i += TEAM) carry[i] = soln[i];
   tm.sync();
@@ -1387,7 +1734,7 @@ __device__ int rk64_cell(const Team<TEAM>& tm, const DevMech& M, const Options& 
     for (int i = tm.lane; i < neq; i += TEAM) error[i] = 0.0;
     tm.sync();
     for (int st = 0; st < 6; st++) {
-      reactor_rhs<TEAM>(tm, M, o.reactor_type, t, soln, ydot, cin.rhoe, cin.rhoesrc, w.src, w.Y, w.sc, w.g, w.qd,
+      reactor_rhs<TEAM, false, TEAM == 1 ? 0 : NS>(tm, M, o.reactor_type, t, soln, ydot, cin.rhoe, cin.rhoesrc, w.src, w.Y, w.sc, w.g, w.qd,
                         w.wdot, w.ei);
       for (int i = tm.lane; i < neq; i += TEAM) {
         error[i] += err[st] * dt_rk * ydot[i];
@@ -1402,9 +1749,9 @@ __device__ int rk64_cell(const Team<TEAM>& tm, const DevMech& M, const Options& 
     for (int i = tm.lane; i < neq; i += TEAM) me = fabs(error[i]) > me ? fabs(error[i]) : me;
     me = tm.max(me);
     if (me < o.atol) {
-      dt_rk = fmin(dt_rk_max, dt_rk * (1.0 * pow((o.atol / me), 0.25)));
+      dt_rk = fmin(dt_rk_max, dt_rk * (1.0 * ppb_pow((o.atol / me), 0.25)));
     } else {
-      dt_rk = fmax(dt_rk_min, dt_rk * (1.0 * pow((o.atol / me), 0.2)));
+      dt_rk = fmax(dt_rk_min, dt_rk * (1.0 * ppb_pow((o.atol / me), 0.2)));
     }
     dt_rk = fmin(dt_rk, dt - t);
   }

@@ -87,8 +87,103 @@ void set_off(const T*& field, size_t off)
 }
 } // namespace
 
-// Species-major gather lists (species -> (reaction, coefficient)) of the
-// productionRate updates, built into the image after the tables.
+// The rate records (RxRate) and the efficiency lists of the third-body and
+// fall-off reactions, in the layouts of DevMech.
+static void pack_rates(const PPBMechTables* t, Packer& pk, DevMech& dm)
+{
+  const int N = t->nsp, R = t->nrxn;
+  auto third = [&](int r) {
+    return t->rx_kind[r] == PPB_RX_THIRD || t->rx_kind[r] == PPB_RX_TROE || t->rx_kind[r] == PPB_RX_LINDEMANN;
+  };
+  int nal = 0, neff = 0;
+  for (int r = 0; r < R; r++) {
+    if (!third(r)) continue;
+    nal++;
+    int n = 0;
+    for (int e = t->eff_off[r]; e < t->eff_off[r + 1]; e++) n += (t->eff_m1[e] != 0.0);
+    neff = n > neff ? n : neff;
+  }
+  neff = (neff + EFF_UNROLL - 1) / EFF_UNROLL * EFF_UNROLL;
+  if (nal > 255 || R > 65535) pk.overflow = true;
+  dm.nal = nal;
+  dm.neff = neff;
+  const size_t off_rr = (pk.used + 15) & ~size_t(15);
+  const size_t off_m1 = off_rr + (size_t)R * sizeof(RxRate);
+  const size_t off_sp = off_m1 + (size_t)neff * nal * sizeof(double);
+  // the slots of a phase space: a repeated species first (see RxRate)
+  auto slots = [&](const int* sp, const double* c, int n, unsigned char (&out)[3]) {
+    int k = 0, runs = 0, repeats = 0;
+    for (int pass = 0; pass < 2; pass++)
+      for (int j = 0; j < n; j++) {
+        const int o = (int)c[j];
+        if ((double)o != c[j] || o < 1) pk.overflow = true;
+        if ((o > 1) != (pass == 0)) continue;
+        runs++;
+        repeats += (o > 1);
+        for (int q = 0; q < o; q++)
+          if (k < 3) out[k++] = (unsigned char)sp[j];
+          else pk.overflow = true;
+      }
+    // a single repeated run is a factor of its own only next to one other
+    // run, or in front of them in species order
+    if (repeats > 1 || (repeats == 1 && runs > 2 && (int)c[0] < 2)) pk.overflow = true;
+    while (k < 3) out[k++] = (unsigned char)N;
+  };
+  int a = 0, fo = 0;
+  for (int r = 0; r < R; r++) {
+    RxRate p;
+    memset(&p, 0, sizeof(p));
+    p.A = t->rx_A[r];
+    p.beta = t->rx_beta[r];
+    p.EaR = t->rx_EaR[r];
+    slots(t->rx_fps_sp + r * PPB_MAXPS, t->rx_fps_c + r * PPB_MAXPS, t->rx_fps_n[r], p.fsp);
+    for (int j = 0; j < 3; j++) p.rsp[j] = (unsigned char)N;
+    for (int j = 0; j < 5; j++) p.kcs[j] = (unsigned char)N;
+    if (t->rx_rev[r]) { // the reverse tables are read for a reversible reaction only
+      slots(t->rx_rps_sp + r * PPB_MAXPS, t->rx_rps_c + r * PPB_MAXPS, t->rx_rps_n[r], p.rsp);
+      if (t->rx_kc_n[r] > 5) pk.overflow = true;
+      for (int j = 0; j < t->rx_kc_n[r] && j < 5; j++) {
+        unsigned long long bits;
+        memcpy(&bits, &t->rx_kc_c[r * PPB_MAXKC + j], 8);
+        if (bits << 16) pk.overflow = true; // more than the top 16 bits of the double
+        p.kcs[j] = (unsigned char)t->rx_kc_sp[r * PPB_MAXKC + j];
+        p.kch[j] = (unsigned short)(bits >> 48);
+      }
+      if (t->rx_kcpow[r] < -1 || t->rx_kcpow[r] > 30) pk.overflow = true;
+    }
+    p.flags = (unsigned char)((t->rx_rev[r] ? RR_REV : 0) | (third(r) ? RR_ALPHA : 0) |
+                              (t->nqss > 0 && t->rx_rmfwd[r] ? RR_RMF : 0) |
+                              ((t->rx_rev[r] ? t->rx_kcpow[r] + 1 : 1) << RR_KCPOW));
+    p.fo = 255;
+    if (t->rx_kind[r] == PPB_RX_TROE || t->rx_kind[r] == PPB_RX_LINDEMANN) p.fo = (unsigned char)fo++;
+    if (third(r)) {
+      int n = 0;
+      for (int e = t->eff_off[r]; e < t->eff_off[r + 1]; e++) {
+        if (t->eff_m1[e] == 0.0) continue;
+        const unsigned char sp = (unsigned char)t->eff_sp[e];
+        pk.put(off_m1 + ((size_t)n * nal + a) * sizeof(double), &t->eff_m1[e], 1);
+        pk.put(off_sp + (size_t)n * nal + a, &sp, 1);
+        n++;
+      }
+      for (; n < neff; n++) {
+        const unsigned char sp = (unsigned char)N;
+        const double z = 0.0;
+        pk.put(off_m1 + ((size_t)n * nal + a) * sizeof(double), &z, 1);
+        pk.put(off_sp + (size_t)n * nal + a, &sp, 1);
+      }
+      p.al = (unsigned char)a++;
+    }
+    for (int w = 0; w < 3; w++)
+      pk.put(off_rr + ((size_t)w * R + r) * 16, reinterpret_cast<const char*>(&p) + 16 * w, 16);
+  }
+  pk.used = off_sp + (size_t)neff * nal;
+  set_off(dm.rr, off_rr);
+  set_off(dm.al_m1, off_m1);
+  set_off(dm.al_sp, off_sp);
+}
+
+// Every table of a mechanism in the layouts of DevMech: the PPBMechTables
+// arrays, then the lists and records derived from them.
 static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
 {
   const int N = t->nsp, R = t->nrxn;
@@ -103,12 +198,45 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
   PPB_ADD(mw, t->mw, N);
   PPB_ADD(imw, t->imw, N);
   PPB_ADD(tmid, t->tmid, NT);
-  PPB_ADD(th_cv, t->th_cv, NT * 10);
-  PPB_ADD(th_cp, t->th_cp, NT * 10);
-  PPB_ADD(th_dcp, t->th_dcp, NT * 8);
-  PPB_ADD(th_u, t->th_u, NT * 12);
-  PPB_ADD(th_h, t->th_h, NT * 12);
-  PPB_ADD(th_g, t->th_g, NT * 14);
+  // thermo polynomials, coefficient-major (th_row, th_at)
+  const int ld = thermo_ld(N);
+  if (NT > ld) pk.overflow = true;
+  auto add_thermo = [&](const double* src, int nc) {
+    const size_t off = (pk.used + 15) & ~size_t(15);
+    for (int k = 0; k < nc; k++)
+      for (int g = 0; g < 2; g++)
+        for (int s = 0; s < ld; s++) {
+          const double v = s < NT ? src[(2 * s + g) * nc + k] : 0.0;
+          pk.put(off + ((size_t)(2 * k + g) * ld + s) * sizeof(double), &v, 1);
+        }
+    pk.used = off + (size_t)2 * nc * ld * sizeof(double);
+    return off;
+  };
+  set_off(dm.th_cv, add_thermo(t->th_cv, 5));
+  set_off(dm.th_cp, add_thermo(t->th_cp, 5));
+  set_off(dm.th_dcp, add_thermo(t->th_dcp, 4));
+  set_off(dm.th_u, add_thermo(t->th_u, 6));
+  set_off(dm.th_h, add_thermo(t->th_h, 6));
+  set_off(dm.th_g, add_thermo(t->th_g, 7));
+  {
+    // e/(RT W) and h/(RT W) at the T solve's bounds
+    const size_t off = (pk.used + 15) & ~size_t(15);
+    const double lim[2] = {90.0, 4000.0};
+    for (int eh = 0; eh < 2; eh++)
+      for (int b = 0; b < 2; b++)
+        for (int s = 0; s < ld; s++) {
+          double v = 0.0;
+          if (s < N) {
+            const double T = lim[b], tm = t->tmid[s];
+            const double* c = (eh ? t->th_h : t->th_u) + (2 * s + ((tm >= 0.0 && T < tm) ? 0 : 1)) * 6;
+            const double T2 = T * T, T3 = T * T * T, T4 = T * T * T * T;
+            v = (c[0] + c[1] * T + c[2] * T2 + c[3] * T3 + c[4] * T4 + c[5] * (1.0 / T)) * t->imw[s];
+          }
+          pk.put(off + ((size_t)(2 * eh + b) * ld + s) * sizeof(double), &v, 1);
+        }
+    pk.used = off + (size_t)4 * ld * sizeof(double);
+    set_off(dm.th_lim, off);
+  }
   PPB_ADD(rx_kind, t->rx_kind, R);
   PPB_ADD(rx_rev, t->rx_rev, R);
   PPB_ADD(rx_kcpow, t->rx_kcpow, R);
@@ -163,25 +291,39 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
 #undef PPB_ADD
   // gather lists, written entry by entry at exact offsets (no temporary
   // containers, so packing itself allocates nothing)
-  int total = 0;
-  for (int r = 0; r < R; r++) total += t->rx_wup_n[r];
-  const size_t off_goff = (pk.used + 15) & ~size_t(15);
-  const size_t off_grx = (off_goff + (N + 1) * sizeof(int) + 15) & ~size_t(15);
-  const size_t off_gc = (off_grx + total * sizeof(int) + 15) & ~size_t(15);
+  int longest = 0;
+  for (int s = 0; s < N; s++) {
+    int cnt = 0;
+    for (int r = 0; r < R; r++)
+      for (int j = 0; j < t->rx_wup_n[r]; j++) cnt += (t->rx_wup_sp[r * PPB_MAXW + j] == s);
+    longest = cnt > longest ? cnt : longest;
+  }
+  const int wgl = (longest + WG_UNROLL - 1) / WG_UNROLL * WG_UNROLL + WG_UNROLL;
+  const size_t off_gn = (pk.used + 15) & ~size_t(15);
+  const size_t off_g = (off_gn + N * sizeof(int) + 15) & ~size_t(15);
   int k = 0;
   for (int s = 0; s < N; s++) {
-    pk.put(off_goff + s * sizeof(int), &k, 1);
+    k = 0;
     for (int r = 0; r < R; r++) {
       for (int j = 0; j < t->rx_wup_n[r]; j++) {
         if (t->rx_wup_sp[r * PPB_MAXW + j] != s) continue;
-        pk.put(off_grx + k * sizeof(int), &r, 1);
-        pk.put(off_gc + k * sizeof(double), &t->rx_wup_c[r * PPB_MAXW + j], 1);
+        unsigned long long bits;
+        memcpy(&bits, &t->rx_wup_c[r * PPB_MAXW + j], 8);
+        if (bits << 16) pk.overflow = true; // more than the top 16 bits of the double
+        const unsigned e = (unsigned)(bits >> 48) << 16 | (unsigned)r;
+        pk.put(off_g + ((size_t)k * N + s) * sizeof(unsigned), &e, 1);
         k++;
       }
     }
+    pk.put(off_gn + s * sizeof(int), &k, 1);
+    for (; k < wgl; k++) {
+      const unsigned e = 0;
+      pk.put(off_g + ((size_t)k * N + s) * sizeof(unsigned), &e, 1);
+    }
   }
-  pk.put(off_goff + N * sizeof(int), &k, 1);
-  pk.used = off_gc + total * sizeof(double);
+  pk.used = off_g + (size_t)wgl * N * sizeof(unsigned);
+  set_off(dm.wg_n, off_gn);
+  set_off(dm.wg, off_g);
   // aJacobian net-stoichiometry gather (species -> (reaction, nu)), reaction order
   int jtotal = 0;
   for (int r = 0; r < R; r++)
@@ -216,7 +358,8 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
     if (t->rx_kind[r] == PPB_RX_THIRD || t->rx_kind[r] == PPB_RX_TROE || t->rx_kind[r] == PPB_RX_LINDEMANN)
       nalpha++;
   const size_t off_fop = off_rxp + (size_t)R * sizeof(RxPack);
-  const size_t off_msk = off_fop + (size_t)nfo * sizeof(FoPack);
+  const size_t off_fow = off_fop + (size_t)nfo * sizeof(FoPack);
+  const size_t off_msk = off_fow + (size_t)nfo * sizeof(FoPack);
   const size_t off_effd = off_msk + (size_t)R * 4 * sizeof(unsigned);
   int fo = 0, aslot = 0;
   for (int r = 0; r < R; r++) {
@@ -314,6 +457,8 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
       f.j3 = (unsigned char)fi[PPB_FOI_J3];
       f.lindemann = (unsigned char)(t->rx_kind[r] == PPB_RX_LINDEMANN);
       pk.put(off_fop + fo * sizeof(FoPack), &f, 1);
+      for (int w = 0; w < 7; w++)
+        pk.put(off_fow + ((size_t)w * nfo + fo) * 16, reinterpret_cast<const char*>(&f) + 16 * w, 16);
       p.fo = (unsigned char)fo++;
     }
     if (t->rx_kind[r] == PPB_RX_THIRD || t->rx_kind[r] == PPB_RX_TROE || t->rx_kind[r] == PPB_RX_LINDEMANN) {
@@ -407,12 +552,12 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
     set_off(dm.al_off, off_aloff);
     set_off(dm.al_rx, off_alrx);
   }
+  dm.nfo = nfo;
+  set_off(dm.fow, off_fow);
   set_off(dm.rxp, off_rxp);
   set_off(dm.fop, off_fop);
   set_off(dm.effmask, off_msk);
-  set_off(dm.wg_off, off_goff);
-  set_off(dm.wg_rx, off_grx);
-  set_off(dm.wg_c, off_gc);
+  pack_rates(t, pk, dm);
   // SRK parameters (zeros for a mechanism without them)
   const double* srk = find_srk(t->name);
   std::vector<double> nosrk;

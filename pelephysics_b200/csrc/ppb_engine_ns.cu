@@ -13,9 +13,9 @@
 namespace ppb {
 
 // ------------------------------------------------------------ react kernels
-template <int NS, int TEAM, typename LT, int METHOD, int RHSV = RHS_IDEAL>
-__device__ void react_one(const Team<TEAM>& tm, const DevMech& M, const Options& o, Work<LT>& w, const Batch& b,
-                          int c, double dt)
+template <int NS, int TEAM, typename LT, int METHOD, int RHSV = RHS_IDEAL, bool UE = false>
+__device__ __forceinline__ void react_one(const Team<TEAM>& tm, const DevMech& M, const Options& o, Work<LT>& w,
+                                          const Batch& b, int c, double dt)
 {
   const int n = NS + 1;
   if (b.mask && b.mask[c] == -1) {
@@ -27,7 +27,7 @@ __device__ void react_one(const Team<TEAM>& tm, const DevMech& M, const Options&
   }
   for (int i = tm.lane; i < n; i += TEAM) {
     const double v = b.y[(size_t)i * b.ld + c];
-    w.zn[0][i] = v;
+    w.zn[i] = v;
     w.y[i] = v;
     w.src[i] = (i < NS) ? b.src[(size_t)i * b.ld + c] : 0.0;
     if (o.use_typ_vals) w.atolv[i] = b.atolv[i];
@@ -36,7 +36,8 @@ __device__ void react_one(const Team<TEAM>& tm, const DevMech& M, const Options&
   const CellIn cin{b.rhoe[c], b.rhoesrc[c]};
   int flag, cost;
   if (METHOD == METHOD_BDF) {
-    Bdf<NS, TEAM, LT, NoRec, RHSV> bdf(tm, M, o, w, cin);
+    NoRec norec;
+    Bdf<NS, TEAM, LT, NoRec, RHSV, UE> bdf(tm, M, o, w, cin, norec);
     flag = bdf.run(dt);
     cost = bdf.s.nfe;
     if (b.stats && tm.lane == 0) {
@@ -50,7 +51,7 @@ __device__ void react_one(const Team<TEAM>& tm, const DevMech& M, const Options&
       st[6] = bdf.ar.ncfn;
     }
   } else {
-    cost = rk64_cell<TEAM, LT>(tm, M, o, w, cin, dt);
+    cost = rk64_cell<NS, TEAM, LT>(tm, M, o, w, cin, dt);
     flag = ST_OK;
     if (b.stats && tm.lane == 0) {
       int* st = b.stats + (size_t)c * 7;
@@ -83,10 +84,8 @@ __global__ void __launch_bounds__(128) k_react_plain(const __grid_constant__ Dev
   Work<double> w;
   {
     double* p = buf;
-    for (int j = 0; j < 6; j++) {
-      w.zn[j] = p;
-      p += n;
-    }
+    w.zn = p;
+    p += 6 * n;
     w.ewt = p; p += n;
     w.acor = p; p += n;
     w.y = p; p += n;
@@ -111,10 +110,31 @@ __global__ void __launch_bounds__(128) k_react_plain(const __grid_constant__ Dev
     w.A = A;
     w.piv = piv;
     w.perm = perm;
+    w.dinv = nullptr; // a team of lanes only
     w.ba = &ba;
   }
   Team<1> tm;
   react_one<NS, 1, double, METHOD>(tm, M, o, w, b, c, dt);
+}
+
+// The team's cells: pulled from the work queue (persistent), or the one at its
+// place in the grid.  One inlined call site of react_one: an out-of-line call
+// would take the workspace's address, which keeps its pointers in local
+// memory and every access through them generic.
+template <int NS, typename LT, int METHOD, int RHSV, bool UE, int TEAM>
+__device__ __forceinline__ void react_cells(const Team<TEAM>& tm, const DevMech& M, const Options& o, Work<LT>& w,
+                                            const Batch& b, double dt, int* queue, int persistent)
+{
+  for (;;) {
+    int c = blockIdx.x * (blockDim.x / TEAM) + threadIdx.x / TEAM;
+    if (persistent) {
+      if (tm.lane == 0) c = atomicAdd(queue, 1);
+      c = tm.bcast_int(c, 0);
+    }
+    if (c >= b.ncells) break;
+    react_one<NS, TEAM, LT, METHOD, RHSV, UE>(tm, M, o, w, b, (persistent && b.order) ? b.order[c] : c, dt);
+    if (!persistent) break;
+  }
 }
 
 // tuned: one team (a warp, or half a warp for small mechanisms) per cell,
@@ -130,19 +150,7 @@ __device__ __forceinline__ void react_team_body(const Team<TEAM>& tm, const DevM
   Work<LT> w;
   carve<LT>(w, smem + (size_t)team * cell_bytes, NS, M.nrxn);
   w.ba = warp_arrays; // one copy of the coefficient arrays per warp of the team
-  const int tpb = blockDim.x / TEAM;
-  if (persistent) {
-    for (;;) {
-      int c = 0;
-      if (tm.lane == 0) c = atomicAdd(queue, 1);
-      c = tm.bcast_int(c, 0);
-      if (c >= b.ncells) break;
-      react_one<NS, TEAM, LT, METHOD>(tm, M, o, w, b, b.order ? b.order[c] : c, dt);
-    }
-  } else {
-    const int c = blockIdx.x * tpb + team;
-    if (c < b.ncells) react_one<NS, TEAM, LT, METHOD>(tm, M, o, w, b, c, dt);
-  }
+  react_cells<NS, LT, METHOD, RHS_IDEAL, false>(tm, M, o, w, b, dt, queue, persistent);
 }
 
 // Warp teams carry no block-shared scratch; a multi-warp team gets 16
@@ -170,22 +178,10 @@ __global__ void __launch_bounds__(MAXT, MINB) k_react_team(const __grid_constant
     } else {
       carve<LT>(w, smem + (size_t)team * cell_bytes, NS, M.nrxn);
     }
-    const int tpb = blockDim.x / TEAM;
-    if (persistent) {
-      __shared__ int rv[3];
-      if (TEAM == 32) w.rv = rendezvous_init(rv, tpb, o.rendezvous);
-      for (;;) {
-        int c = 0;
-        if (tm.lane == 0) c = atomicAdd(queue, 1);
-        c = __shfl_sync(tm.mask, c, 0, TEAM);
-        if (c >= b.ncells) break;
-        react_one<NS, TEAM, LT, METHOD, RHSV>(tm, M, o, w, b, b.order ? b.order[c] : c, dt);
-      }
-      rendezvous_leave(w.rv);
-    } else {
-      const int c = blockIdx.x * tpb + team;
-      if (c < b.ncells) react_one<NS, TEAM, LT, METHOD, RHSV>(tm, M, o, w, b, c, dt);
-    }
+    __shared__ int rv[3];
+    if (TEAM == 32 && persistent) w.rv = rendezvous_init(rv, blockDim.x / TEAM, o.rendezvous);
+    react_cells<NS, LT, METHOD, RHSV, MAXT == 512 && RHSV == RHS_IDEAL>(tm, M, o, w, b, dt, queue, persistent);
+    rendezvous_leave(w.rv);
   }
 }
 

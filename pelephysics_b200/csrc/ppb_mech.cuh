@@ -28,6 +28,7 @@ namespace ppb {
 static __device__ PPB_MATH_ATTR double ppb_exp(double x) { return ::exp(x); }
 static __device__ PPB_MATH_ATTR double ppb_log(double x) { return ::log(x); }
 static __device__ PPB_MATH_ATTR double ppb_log10(double x) { return ::log10(x); }
+static __device__ PPB_MATH_ATTR double ppb_pow(double x, double y) { return ::pow(x, y); }
 
 
 constexpr double RU = 8.31446261815324e7; // erg/(mol K), PhysicsConstants.H:11
@@ -37,8 +38,16 @@ constexpr double RU = 8.31446261815324e7; // erg/(mol K), PhysicsConstants.H:11
 struct DevMech {
   int nsp, nrxn;
   int nqss, nrq; // QSS species and reactions with one (PPBMechTables)
+  int nfo, nal, neff; // fall-off reactions, third-body and fall-off reactions, the longest list of efficiencies
+  int pad_;
   const double *mw, *imw, *tmid;
+  // NASA-7 polynomials, coefficient-major: coefficient k of range g (0 below
+  // tmid) of species s at [(2 k + g) * thermo_ld(nsp) + s], so that lanes
+  // owning consecutive species load consecutive doubles
   const double *th_cv, *th_cp, *th_dcp, *th_u, *th_h, *th_g;
+  // e_k / (RT W_k) (then h_k) of species k at the bounds of the T solve:
+  // [u at 90 K | u at 4000 K | h at 90 K | h at 4000 K], thermo_ld(nsp) each
+  const double* th_lim;
   const int *rx_kind, *rx_rev, *rx_kcpow;
   const double *rx_A, *rx_beta, *rx_EaR, *rx_sum_nuk;
   const int *fps_n, *fps_sp;
@@ -59,10 +68,20 @@ struct DevMech {
   const double *eff_e, *eff_m1;
   const double* fo_d;
   const int* fo_i;
-  // species-major gather of the productionRate updates: for species s,
-  // entries g in [wg_off[s], wg_off[s+1]) add wg_c[g] * qdot[wg_rx[g]]
-  const int *wg_off, *wg_rx;
-  const double* wg_c;
+  // gather of the productionRate updates: species s adds, in reaction order,
+  // c qdot[r] for entries wg[j nsp + s], j < wg_n[s]: the top 16 bits of the
+  // double c, then the reaction r in 16 bits (padded to the longest list,
+  // rounded up to WG_UNROLL, and WG_UNROLL entries more)
+  const int* wg_n;
+  const unsigned* wg;
+  // the rate records (RxRate) word by word: word w of reaction r at
+  // rr[w nrxn + r]; the fall-off records (FoPack) likewise, word w of record
+  // f at fow[w nfo + f]; efficiency j of third-body reaction a at
+  // [j nal + a] (eff - 1 and the species, padded with 0 and the unit slot to
+  // neff, a multiple of EFF_UNROLL)
+  const int4 *rr, *fow;
+  const double* al_m1;
+  const unsigned char* al_sp;
   // packed per-reaction records (see RxPack) for the warp-cooperative paths
   const struct RxPack* rxp;
   const struct FoPack* fop;
@@ -114,6 +133,30 @@ struct alignas(16) RxPack {
   unsigned char pad;
 };
 static_assert(sizeof(RxPack) == 80, "RxPack is five 16-byte words");
+
+// What a rate evaluation needs of one reaction, in 48 bytes (three 16-byte
+// words, stored word-major so that a warp's loads are contiguous: the 80-byte
+// records above, read by consecutive lanes, took 20 cache lines per load).
+// Phase spaces are at most three slots (checked when the tables are packed),
+// a repeated species first, so that the left-to-right product of the slots is
+// the product of the species' powers in species order, bit for bit.
+struct alignas(16) RxRate {
+  double A, beta, EaR;
+  unsigned char fsp[3], rsp[3];
+  unsigned char kcs[5];
+  unsigned char flags;   // RR_REV, RR_ALPHA, RR_RMF, and kcpow + 1 from bit RR_KCPOW
+  unsigned short kch[5]; // top 16 bits of the double coefficient of kcs
+  unsigned char fo;      // fall-off record, 255 = none
+  unsigned char al;      // third-body slot (al_m1, al_sp)
+};
+static_assert(sizeof(RxRate) == 48, "RxRate is three 16-byte words");
+enum { RR_REV = 1, RR_ALPHA = 2, RR_RMF = 4, RR_KCPOW = 3 };
+constexpr int WG_UNROLL = 8;  // gather entries loaded together
+constexpr int EFF_UNROLL = 4; // efficiencies loaded together
+
+// Leading dimension of the thermo tables: the species, then (QSS mechanisms)
+// the unit slot and at most ten QSS species, rounded up to 32 bytes.
+__host__ __device__ constexpr int thermo_ld(int nsp) { return (nsp + 11 + 3) & ~3; }
 
 struct alignas(16) FoPack {
   double P0, k0, beta0, EaR0, prdim, a, T3, T1, T2, oma, iT3, iT1;
@@ -190,6 +233,78 @@ struct Team : TeamScratch<TEAM> {
     } else {
       return reduce(x, [](double a, double b) { return a + b; });
     }
+  }
+  // Two (four) sums at once, each the same bits as sum(): the xor butterfly
+  // adds the same pairs whichever lane does it, so after the first level(s)
+  // every lane carries on with one of the values only, and the results are
+  // broadcast at the end (32 lanes, four sums: 10 double shuffles and 6
+  // additions a lane instead of 20 and 20).
+  __device__ __forceinline__ void sum2(double& a, double& b) const
+  {
+    if constexpr (TEAM == 32 || TEAM == 16) {
+      constexpr int H = TEAM / 2;
+      const bool hi = (lane & H) != 0;
+      double x = hi ? b : a;
+      x += __shfl_xor_sync(mask, hi ? a : b, H, TEAM);
+#pragma unroll
+      for (int o = H / 2; o > 0; o >>= 1) x += __shfl_xor_sync(mask, x, o, TEAM);
+      a = __shfl_sync(mask, x, 0, TEAM);
+      b = __shfl_sync(mask, x, H, TEAM);
+    } else if constexpr (TEAM > 32) {
+      double v[2] = {a, b};
+      sum_multi<2>(v);
+      a = v[0];
+      b = v[1];
+    }
+  }
+  __device__ __forceinline__ void sum4(double& a, double& b, double& c, double& d) const
+  {
+    if constexpr (TEAM == 32 || TEAM == 16) {
+      constexpr int H = TEAM / 2, Q = TEAM / 4;
+      const bool hi = (lane & H) != 0, hq = (lane & Q) != 0;
+      double x = hi ? c : a, y = hi ? d : b;
+      x += __shfl_xor_sync(mask, hi ? a : c, H, TEAM);
+      y += __shfl_xor_sync(mask, hi ? b : d, H, TEAM);
+      double z = hq ? y : x;
+      z += __shfl_xor_sync(mask, hq ? x : y, Q, TEAM);
+#pragma unroll
+      for (int o = Q / 2; o > 0; o >>= 1) z += __shfl_xor_sync(mask, z, o, TEAM);
+      a = __shfl_sync(mask, z, 0, TEAM);
+      b = __shfl_sync(mask, z, Q, TEAM);
+      c = __shfl_sync(mask, z, H, TEAM);
+      d = __shfl_sync(mask, z, H + Q, TEAM);
+    } else if constexpr (TEAM > 32) {
+      double v[4] = {a, b, c, d};
+      sum_multi<4>(v);
+      a = v[0];
+      b = v[1];
+      c = v[2];
+      d = v[3];
+    }
+  }
+  // several sums of a multi-warp team behind one pair of barriers
+  template <int K>
+  __device__ __forceinline__ void sum_multi(double (&v)[K]) const
+  {
+    static_assert(TEAM > 32, "multi-warp teams");
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+    if ((lane & 31) == 0) {
+#pragma unroll
+      for (int k = 0; k < K; k++) this->red[k * NW + (lane >> 5)] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      double x = this->red[k * NW];
+#pragma unroll
+      for (int i = 1; i < NW; i++) x += this->red[k * NW + i];
+      v[k] = x;
+    }
+    __syncthreads();
   }
   __device__ __forceinline__ double max(double x) const
   {
@@ -282,50 +397,71 @@ __device__ __forceinline__ int nasa_range(const DevMech& M, int s, double T)
   return (tm >= 0.0 && T < tm) ? 0 : 1;
 }
 
-// mechanism.H cv_R (thermo.py:516-526)
-__device__ __forceinline__ double cv_R(const DevMech& M, int s, double T)
+// Coefficient k of species s at T: th_at(row, k) with row = th_row(table, s, T).
+// NS > 0 makes the table's stride a compile-time constant.
+template <int NS = 0>
+__device__ __forceinline__ const double* th_row(const DevMech& M, const double* tab, int s, double T)
 {
-  const double* c = M.th_cv + (2 * s + nasa_range(M, s, T)) * 5;
+  const int ld = NS > 0 ? thermo_ld(NS) : thermo_ld(M.nsp);
+  return tab + (nasa_range(M, s, T) ? ld : 0) + s;
+}
+template <int NS = 0>
+__device__ __forceinline__ double th_at(const DevMech& M, const double* row, int k)
+{
+  const int ld = NS > 0 ? thermo_ld(NS) : thermo_ld(M.nsp);
+  return __ldg(row + 2 * ld * k);
+}
+
+// cv/R or cp/R: the quartic both share (tab = th_cv or th_cp; mechanism.H
+// cv_R, cp_R, thermo.py:516-559)
+template <int NS = 0>
+__device__ __forceinline__ double c_R(const DevMech& M, const double* tab, int s, double T)
+{
+  const double* c = th_row<NS>(M, tab, s, T);
   const double T2 = T * T, T3 = T * T * T, T4 = T * T * T * T;
-  return __ldg(c) + __ldg(c + 1) * T + __ldg(c + 2) * T2 + __ldg(c + 3) * T3 + __ldg(c + 4) * T4;
+  return th_at<NS>(M, c, 0) + th_at<NS>(M, c, 1) * T + th_at<NS>(M, c, 2) * T2 + th_at<NS>(M, c, 3) * T3 +
+         th_at<NS>(M, c, 4) * T4;
 }
-// mechanism.H cp_R (thermo.py:549-559)
-__device__ __forceinline__ double cp_R(const DevMech& M, int s, double T)
+// e/RT or h/RT (tab = th_u or th_h; mechanism.H speciesInternalEnergy,
+// speciesEnthalpy, thermo.py:625-669)
+template <int NS = 0>
+__device__ __forceinline__ double e_RT(const DevMech& M, const double* tab, int s, double T, double invT)
 {
-  const double* c = M.th_cp + (2 * s + nasa_range(M, s, T)) * 5;
+  const double* c = th_row<NS>(M, tab, s, T);
   const double T2 = T * T, T3 = T * T * T, T4 = T * T * T * T;
-  return __ldg(c) + __ldg(c + 1) * T + __ldg(c + 2) * T2 + __ldg(c + 3) * T3 + __ldg(c + 4) * T4;
+  return th_at<NS>(M, c, 0) + th_at<NS>(M, c, 1) * T + th_at<NS>(M, c, 2) * T2 + th_at<NS>(M, c, 3) * T3 +
+         th_at<NS>(M, c, 4) * T4 + th_at<NS>(M, c, 5) * invT;
 }
-// mechanism.H dcvpRdT (thermo.py:561-570)
-__device__ __forceinline__ double dcvpRdT(const DevMech& M, int s, double T)
-{
-  const double* c = M.th_dcp + (2 * s + nasa_range(M, s, T)) * 4;
-  const double T2 = T * T, T3 = T * T * T;
-  return __ldg(c) + __ldg(c + 1) * T + __ldg(c + 2) * T2 + __ldg(c + 3) * T3;
-}
-// mechanism.H speciesInternalEnergy, e/RT (thermo.py:625-646)
+template <int NS = 0>
+__device__ __forceinline__ double cv_R(const DevMech& M, int s, double T) { return c_R<NS>(M, M.th_cv, s, T); }
+template <int NS = 0>
+__device__ __forceinline__ double cp_R(const DevMech& M, int s, double T) { return c_R<NS>(M, M.th_cp, s, T); }
+template <int NS = 0>
 __device__ __forceinline__ double u_RT(const DevMech& M, int s, double T, double invT)
 {
-  const double* c = M.th_u + (2 * s + nasa_range(M, s, T)) * 6;
-  const double T2 = T * T, T3 = T * T * T, T4 = T * T * T * T;
-  return __ldg(c) + __ldg(c + 1) * T + __ldg(c + 2) * T2 + __ldg(c + 3) * T3 + __ldg(c + 4) * T4 +
-         __ldg(c + 5) * invT;
+  return e_RT<NS>(M, M.th_u, s, T, invT);
 }
-// mechanism.H speciesEnthalpy, h/RT (thermo.py:649-669)
+template <int NS = 0>
 __device__ __forceinline__ double h_RT(const DevMech& M, int s, double T, double invT)
 {
-  const double* c = M.th_h + (2 * s + nasa_range(M, s, T)) * 6;
-  const double T2 = T * T, T3 = T * T * T, T4 = T * T * T * T;
-  return __ldg(c) + __ldg(c + 1) * T + __ldg(c + 2) * T2 + __ldg(c + 3) * T3 + __ldg(c + 4) * T4 +
-         __ldg(c + 5) * invT;
+  return e_RT<NS>(M, M.th_h, s, T, invT);
+}
+// mechanism.H dcvpRdT (thermo.py:561-570)
+template <int NS = 0>
+__device__ __forceinline__ double dcvpRdT(const DevMech& M, int s, double T)
+{
+  const double* c = th_row<NS>(M, M.th_dcp, s, T);
+  const double T2 = T * T, T3 = T * T * T;
+  return th_at<NS>(M, c, 0) + th_at<NS>(M, c, 1) * T + th_at<NS>(M, c, 2) * T2 + th_at<NS>(M, c, 3) * T3;
 }
 // mechanism.H gibbs, g/RT (thermo.py:572-595)
+template <int NS = 0>
 __device__ __forceinline__ double g_RT(const DevMech& M, int s, double T, double invT, double logT)
 {
-  const double* c = M.th_g + (2 * s + nasa_range(M, s, T)) * 7;
+  const double* c = th_row<NS>(M, M.th_g, s, T);
   const double T2 = T * T, T3 = T * T * T, T4 = T * T * T * T;
-  return __ldg(c) * invT + __ldg(c + 1) + __ldg(c + 2) * logT + __ldg(c + 3) * T + __ldg(c + 4) * T2 +
-         __ldg(c + 5) * T3 + __ldg(c + 6) * T4;
+  return th_at<NS>(M, c, 0) * invT + th_at<NS>(M, c, 1) + th_at<NS>(M, c, 2) * logT + th_at<NS>(M, c, 3) * T +
+         th_at<NS>(M, c, 4) * T2 + th_at<NS>(M, c, 5) * T3 + th_at<NS>(M, c, 6) * T4;
 }
 
 // Mixture energy (EH=0: CKUBMS, erg/g) or enthalpy (EH=1: CKHBMS) and the
@@ -339,11 +475,10 @@ __device__ __forceinline__ void mix_e_c(
   for (int s = tm.lane; s < M.nsp; s += TEAM) {
     const double im = __ldg(M.imw + s);
     const double ys = Y[s];
-    se += ys * (EH ? h_RT(M, s, T, invT) : u_RT(M, s, T, invT)) * im;
-    sc += ys * (EH ? cp_R(M, s, T) : cv_R(M, s, T)) * im;
+    se += ys * e_RT(M, EH ? M.th_h : M.th_u, s, T, invT) * im;
+    sc += ys * c_R(M, EH ? M.th_cp : M.th_cv, s, T) * im;
   }
-  se = tm.sum(se);
-  sc = tm.sum(sc);
+  tm.sum2(se, sc);
   const double RT = RU * T;
   e = se * RT;
   c = sc * RU;
@@ -355,7 +490,7 @@ __device__ __forceinline__ double mix_e(const Team<TEAM>& tm, const DevMech& M, 
   const double invT = 1.0 / T;
   double se = 0.0;
   for (int s = tm.lane; s < M.nsp; s += TEAM) {
-    se += Y[s] * (EH ? h_RT(M, s, T, invT) : u_RT(M, s, T, invT)) * __ldg(M.imw + s);
+    se += Y[s] * e_RT(M, EH ? M.th_h : M.th_u, s, T, invT) * __ldg(M.imw + s);
   }
   se = tm.sum(se);
   return se * (RU * T);
@@ -366,49 +501,77 @@ __device__ __forceinline__ double mix_c(const Team<TEAM>& tm, const DevMech& M, 
 {
   double sc = 0.0;
   for (int s = tm.lane; s < M.nsp; s += TEAM) {
-    sc += Y[s] * (EH ? cp_R(M, s, T) : cv_R(M, s, T)) * __ldg(M.imw + s);
+    sc += Y[s] * c_R(M, EH ? M.th_cp : M.th_cv, s, T) * __ldg(M.imw + s);
   }
   sc = tm.sum(sc);
   return sc * RU;
 }
 
+// The species of a lane at the temperature a T solve ended at: the mixture's
+// sum of Y_k c_k / W_k and, for one species per lane, its e_k/RT (h_k/RT).
+struct ThermoAtT {
+  bool have = false; // filled (the solve ended in its Newton iteration)
+  double csum = 0.0, e = 0.0;
+};
+
+// The energy e of a T solve as the product a b it was rounded from: with use,
+// the Newton differences take it unrounded, fma(a, b, -e(T)).
+struct EnergyProduct {
+  double a, b;
+  bool use;
+};
+
 // mechanism.H GET_T_GIVEN_EY / GET_T_GIVEN_HY: Newton from the supplied T,
 // |step| <= 100 K, stop at |dT| < 1e-6 K, <= 200 iterations, linear
-// extrapolation outside [90, 4000] K (returns 1 there).  When the supplied T
-// lies in [90, 4000] K (the integrator's case: it is the previous T), the
-// bounds' energies and the first Newton iterate's energy and heat capacity
-// are summed in one pass over the species; every sum is formed in the order
-// mix_e / mix_e_c form it.
-template <int TEAM>
-__device__ int t_from_energy(const Team<TEAM>& tm, const DevMech& M, int EH, double e, const double* Y, double& t)
+// extrapolation outside [90, 4000] K (returns 1 there).  The bounds' energies
+// come from tables (th_lim) and are summed with the first iterate's energy and
+// heat capacity; every other sum is formed in the order mix_e / mix_e_c form
+// it.  The last iterate's heat-capacity sum and species energies are what a
+// caller would evaluate again at the final T (same formulas, same T): they
+// are handed out in *at.
+template <int TEAM, int NS = 0>
+__device__ __forceinline__ int t_from_energy(const Team<TEAM>& tm, const DevMech& M, int EH, double e,
+                                             const double* Y, double& t, ThermoAtT* at = nullptr,
+                                             const EnergyProduct* ep = nullptr)
 {
+  constexpr bool ONE = NS > 0 && NS <= TEAM; // one species per lane
+  const int N = NS > 0 ? NS : M.nsp;
+  const int ld = thermo_ld(N);
   const double tmin = 90, tmax = 4000;
+  const double* te = EH ? M.th_h : M.th_u;
+  const double* tc = EH ? M.th_cp : M.th_cv;
+  const double* lim = M.th_lim + (EH ? 2 * ld : 0);
   double t1 = t;
-  double emin, emax, e1 = 0.0, cv1 = 0.0;
+  double smin = 0.0, smax = 0.0, se = 0.0, sc = 0.0, el = 0.0;
+  double yl = 0.0, iml = 0.0;
   const bool fused = !(t1 < tmin || t1 > tmax);
-  if (fused) {
-    const double imin = 1.0 / tmin, imax = 1.0 / tmax, i1 = 1.0 / t1;
-    double smin = 0.0, smax = 0.0, se = 0.0, sc = 0.0;
-    for (int s = tm.lane; s < M.nsp; s += TEAM) {
+  const double i1 = 1.0 / t1;
+  if constexpr (ONE) {
+    if (tm.lane < N) {
+      yl = Y[tm.lane];
+      iml = __ldg(M.imw + tm.lane);
+      smin += yl * __ldg(lim + tm.lane);
+      smax += yl * __ldg(lim + ld + tm.lane);
+      if (fused) {
+        el = e_RT<NS>(M, te, tm.lane, t1, i1);
+        se += yl * el * iml;
+        sc += yl * c_R<NS>(M, tc, tm.lane, t1) * iml;
+      }
+    }
+  } else {
+    for (int s = tm.lane; s < N; s += TEAM) {
       const double im = __ldg(M.imw + s);
       const double ys = Y[s];
-      smin += Y[s] * (EH ? h_RT(M, s, tmin, imin) : u_RT(M, s, tmin, imin)) * im;
-      smax += Y[s] * (EH ? h_RT(M, s, tmax, imax) : u_RT(M, s, tmax, imax)) * im;
-      se += ys * (EH ? h_RT(M, s, t1, i1) : u_RT(M, s, t1, i1)) * im;
-      sc += ys * (EH ? cp_R(M, s, t1) : cv_R(M, s, t1)) * im;
+      smin += ys * __ldg(lim + s);
+      smax += ys * __ldg(lim + ld + s);
+      if (fused) {
+        se += ys * e_RT<NS>(M, te, s, t1, i1) * im;
+        sc += ys * c_R<NS>(M, tc, s, t1) * im;
+      }
     }
-    smin = tm.sum(smin);
-    smax = tm.sum(smax);
-    se = tm.sum(se);
-    sc = tm.sum(sc);
-    emin = smin * (RU * tmin);
-    emax = smax * (RU * tmax);
-    e1 = se * (RU * t1);
-    cv1 = sc * RU;
-  } else {
-    emin = mix_e(tm, M, EH, tmin, Y);
-    emax = mix_e(tm, M, EH, tmax, Y);
   }
+  tm.sum4(smin, smax, se, sc);
+  const double emin = smin * (RU * tmin), emax = smax * (RU * tmax);
   if (e < emin) {
     t = tmin - (emin - e) / mix_c(tm, M, EH, tmin, Y);
     return 1;
@@ -418,25 +581,48 @@ __device__ int t_from_energy(const Team<TEAM>& tm, const DevMech& M, int EH, dou
     return 1;
   }
   if (!fused) t1 = tmin + (tmax - tmin) / (emax - emin) * (e - emin);
+  bool conv = false;
   for (int i = 0; i < 200; ++i) {
-    double ec, cv;
-    if (i == 0 && fused) {
-      ec = e1;
-      cv = cv1;
-    } else {
-      mix_e_c(tm, M, EH, t1, Y, ec, cv);
+    if (i > 0 || !fused) {
+      const double invT = 1.0 / t1;
+      se = 0.0;
+      sc = 0.0;
+      if constexpr (ONE) {
+        if (tm.lane < N) {
+          el = e_RT<NS>(M, te, tm.lane, t1, invT);
+          se += yl * el * iml;
+          sc += yl * c_R<NS>(M, tc, tm.lane, t1) * iml;
+        }
+      } else {
+        for (int s = tm.lane; s < N; s += TEAM) {
+          const double im = __ldg(M.imw + s);
+          const double ys = Y[s];
+          se += ys * e_RT<NS>(M, te, s, t1, invT) * im;
+          sc += ys * c_R<NS>(M, tc, s, t1) * im;
+        }
+      }
+      tm.sum2(se, sc);
     }
-    double dt = (e - ec) / cv;
+    // (rounded product, then the difference: no contraction, whatever the
+    // code around it)
+    const double ec = __dmul_rn(se, RU * t1), cv = sc * RU;
+    double dt = (ep && ep->use ? __fma_rn(ep->a, ep->b, -ec) : __dsub_rn(e, ec)) / cv;
     if (dt > 100.) {
       dt = 100.;
     } else if (dt < -100.) {
       dt = -100.;
     } else if (fabs(dt) < 1.e-6) {
+      conv = true;
       break;
     }
     t1 += dt;
   }
   t = t1;
+  if (at) {
+    at->have = conv;
+    at->csum = sc;
+    at->e = el;
+  }
   return 0;
 }
 
@@ -455,9 +641,10 @@ __device__ __forceinline__ double phase_space(const int* sp, const double* c, in
 
 __device__ __forceinline__ double refc_pow(int p, double refC, double refCinv)
 {
-  double r = 1.0;
-  for (int q = 0; q < p; q++) r *= refCinv;
-  for (int q = 0; q < -p; q++) r *= refC;
+  if (p == 0) return 1.0;
+  const double b = p > 0 ? refCinv : refC;
+  double r = b;
+  for (int q = p > 0 ? p : -p; q > 1; q--) r *= b;
   return r;
 }
 
@@ -622,25 +809,46 @@ __device__ __forceinline__ bool slots_has(const unsigned char (&sp)[K], int k)
   return h;
 }
 
-// Rates of progress q_f, q_r from a packed record (same formulas as
-// rxn_qdot).
-__device__ __forceinline__ void rx_rates_packed(
-  const DevMech& M, const RxPack& p, double T, double invT, double logT, double refC, double refCinv, double mixture,
-  const double* sc, const double* g, double& qf_out, double& qr_out)
+// The rate record of reaction r (word-major: consecutive lanes read
+// consecutive 16-byte words).
+__device__ __forceinline__ RxRate load_rr(const DevMech& M, int r)
 {
-  const int kind = p.kind;
+  RxRate p;
+  int4* dst = reinterpret_cast<int4*>(&p);
+#pragma unroll
+  for (int i = 0; i < 3; i++) dst[i] = __ldg(M.rr + i * M.nrxn + r);
+  return p;
+}
+
+__device__ __forceinline__ FoPack load_fow(const DevMech& M, int f)
+{
+  FoPack p;
+  int4* dst = reinterpret_cast<int4*>(&p);
+#pragma unroll
+  for (int i = 0; i < 7; i++) dst[i] = __ldg(M.fow + i * M.nfo + f);
+  return p;
+}
+
+// Rates of progress q_f, q_r from a rate record (same formulas as rxn_qdot).
+__device__ __forceinline__ void rr_rates(const DevMech& M, const RxRate& p, double T, double invT, double logT,
+                                         double refC, double refCinv, double mixture, const double* sc,
+                                         const double* g, double& qf_out, double& qr_out)
+{
   const double k_f = p.A * ppb_exp(p.beta * logT - p.EaR * invT);
   double Corr = 1.0;
-  const bool corr = (kind == PPB_RX_THIRD || kind == PPB_RX_TROE || kind == PPB_RX_LINDEMANN);
+  const bool corr = (p.flags & RR_ALPHA) != 0;
   if (corr) {
     Corr = mixture;
-    for (int e = p.eff0; e < p.eff0 + p.effn; e++) {
-      const double m1 = __ldg(M.eff_m1 + e);
-      if (m1 != 0.0) Corr += m1 * sc[__ldg(M.eff_sp + e)];
+    for (int j = 0; j < M.neff; j += EFF_UNROLL) {
+#pragma unroll
+      for (int q = 0; q < EFF_UNROLL; q++) {
+        const int e = (j + q) * M.nal + p.al;
+        Corr += __ldg(M.al_m1 + e) * sc[__ldg(M.al_sp + e)];
+      }
     }
   }
   if (p.fo != 255) {
-    const FoPack f = load_fo(M, p.fo);
+    const FoPack f = load_fow(M, p.fo);
     const double redP = Corr / k_f * f.P0 * ppb_exp(f.beta0 * logT - f.EaR0 * invT);
     const double F = redP / (1.0 + redP);
     if (!f.lindemann) {
@@ -659,28 +867,18 @@ __device__ __forceinline__ void rx_rates_packed(
       Corr = F;
     }
   }
-  const double phf = slots_product(p.fsp, sc);
+  const double phf = (sc[p.fsp[0]] * sc[p.fsp[1]]) * sc[p.fsp[2]];
   const double qf = corr ? Corr * k_f * phf : k_f * phf;
   double qr = 0.0;
-  if (p.rev) {
+  if (p.flags & RR_REV) {
     double arg = 0.0;
 #pragma unroll
-    for (int j = 0; j < 6; j++) arg += (double)p.kcc[j] * g[p.kcs[j]];
-    const double phr = slots_product(p.rsp, sc);
-    qr = (corr ? Corr * k_f : k_f) * ppb_exp(-arg) * refc_pow(p.kcpow, refC, refCinv) * phr;
+    for (int j = 0; j < 5; j++) arg += __hiloint2double((int)((unsigned)p.kch[j] << 16), 0) * g[p.kcs[j]];
+    const double phr = (sc[p.rsp[0]] * sc[p.rsp[1]]) * sc[p.rsp[2]];
+    qr = (corr ? Corr * k_f : k_f) * ppb_exp(-arg) * refc_pow((p.flags >> RR_KCPOW) - 1, refC, refCinv) * phr;
   }
-  qf_out = p.rmf ? 0.0 : qf;
+  qf_out = (p.flags & RR_RMF) ? 0.0 : qf;
   qr_out = qr;
-}
-
-// Net rate of progress from a packed record.
-__device__ __forceinline__ double rx_qdot_packed(
-  const DevMech& M, const RxPack& p, double T, double invT, double logT, double refC, double refCinv, double mixture,
-  const double* sc, const double* g)
-{
-  double qf, qr;
-  rx_rates_packed(M, p, T, invT, logT, refC, refCinv, mixture, sc, g, qf, qr);
-  return qf - qr;
 }
 
 // Scratch doubles of the QSS solve: the coefficients q_f,k, q_r,k (2 nrq)
@@ -713,9 +911,9 @@ __device__ void qss_solve(const Team<TEAM>& tm, const DevMech& M, double* sc, do
   }
   tm.sync();
   for (int k = tm.lane; k < K; k += TEAM) {
-    const RxPack p = load_rx(M, __ldg(M.q_rx + k));
+    const RxRate p = load_rr(M, __ldg(M.q_rx + k));
     double qf, qr;
-    rx_rates_packed(M, p, T, invT, logT, refC, refCinv, mixture, sc, g, qf, qr);
+    rr_rates(M, p, T, invT, logT, refC, refCinv, mixture, sc, g, qf, qr);
     co[2 * k] = qf;
     co[2 * k + 1] = qr;
   }
@@ -775,25 +973,53 @@ struct RateScratch {
   double* qco = nullptr; // QSS scratch (qss_scratch_doubles), for a QSS mechanism
 };
 
+// wdot of species s from the net rates, in reaction order.  WG_UNROLL entries
+// are loaded together (the padding entries are loaded, not added).
+__device__ __forceinline__ double rate_gather(const DevMech& M, int N, int s, const double* qd)
+{
+  double w = 0.0;
+  const int cnt = __ldg(M.wg_n + s);
+  const unsigned* pw = M.wg + s;
+  unsigned e[WG_UNROLL];
+#pragma unroll
+  for (int i = 0; i < WG_UNROLL; i++) e[i] = __ldg(pw + i * N);
+  for (int j = 0; j < cnt; j += WG_UNROLL) {
+    double c[WG_UNROLL], q[WG_UNROLL];
+#pragma unroll
+    for (int i = 0; i < WG_UNROLL; i++) {
+      c[i] = __hiloint2double((int)(e[i] & 0xffff0000u), 0);
+      q[i] = qd[e[i] & 0xffffu];
+    }
+    // the next entries while these are summed (the list ends with a group of
+    // padding)
+#pragma unroll
+    for (int i = 0; i < WG_UNROLL; i++) e[i] = __ldg(pw + (j + WG_UNROLL + i) * N);
+#pragma unroll
+    for (int i = 0; i < WG_UNROLL; i++) {
+      const double v = __fma_rn(c[i], q[i], w);
+      w = j + i < cnt ? v : w;
+    }
+  }
+  return w;
+}
+
 // The reactions and the species gather of productionRate for a team of
 // lanes (TEAM > 1), given g/RT in rs.g (0 in the padding slot), sc with 1 in
 // its padding slot, and the temperature terms and mixture concentration.
-template <int TEAM>
+template <int TEAM, int NS = 0>
 __device__ __forceinline__ void production_rate_core(const Team<TEAM>& tm, const DevMech& M, double* wdot,
                                                      const double* sc_in, double T, double invT, double logT,
                                                      double refC, double refCinv, double mixture, RateScratch& rs)
 {
+  const int N = NS > 0 ? NS : M.nsp;
   for (int r = tm.lane; r < M.nrxn; r += TEAM) {
-    const RxPack p = load_rx(M, r);
-    rs.qd[r] = rx_qdot_packed(M, p, T, invT, logT, refC, refCinv, mixture, sc_in, rs.g);
+    const RxRate p = load_rr(M, r);
+    double qf, qr;
+    rr_rates(M, p, T, invT, logT, refC, refCinv, mixture, sc_in, rs.g, qf, qr);
+    rs.qd[r] = __dsub_rn(qf, qr); // both rounded: no contraction with either product
   }
   tm.sync();
-  for (int s = tm.lane; s < M.nsp; s += TEAM) {
-    double w = 0.0;
-    const int g1 = __ldg(M.wg_off + s + 1);
-    for (int gi = __ldg(M.wg_off + s); gi < g1; gi++) w += __ldg(M.wg_c + gi) * rs.qd[__ldg(M.wg_rx + gi)];
-    wdot[s] = w;
-  }
+  for (int s = tm.lane; s < N; s += TEAM) wdot[s] = rate_gather(M, N, s, rs.qd);
   tm.sync();
 }
 

@@ -53,7 +53,7 @@ template <typename LT>
 __host__ __device__ inline size_t team_bytes(int N, int R, int Q = 0, int K = 0)
 {
   const int n = N + 1;
-  const size_t d = 22 * (size_t)n + (size_t)R;
+  const size_t d = 23 * (size_t)n + (size_t)R;
   size_t b = d * 8 + j_region_bytes<LT>(N) + jx_region_bytes<LT>(R) + a_region_bytes<LT>(N, R) +
              ((8 * (size_t)n + 7) & ~size_t(7)) + sizeof(BdfArrays);
   b = (b + 15) & ~size_t(15);
@@ -67,10 +67,8 @@ __device__ inline void carve(Work<LT>& w, char* base, int N, int R, int Q = 0, i
 {
   const int n = N + 1;
   double* p = (double*)base;
-  for (int j = 0; j < 6; j++) {
-    w.zn[j] = p;
-    p += n;
-  }
+  w.zn = p;
+  p += 6 * n;
   w.ewt = p; p += n;
   w.acor = p; p += n;
   w.y = p; p += n;
@@ -87,6 +85,7 @@ __device__ inline void carve(Work<LT>& w, char* base, int N, int R, int Q = 0, i
   w.h1 = p; p += n;
   w.h2 = p; p += n;
   w.h3 = p; p += n;
+  w.dinv = p; p += n;
   w.qd = p; p += R;
   char* q = (char*)p;
   if constexpr (sizeof(LT) == sizeof(double)) {
