@@ -75,10 +75,31 @@ __device__ __forceinline__ long view_off(const BoxView& v, int i, int j, int k)
   return (long)(i - v.lo[0]) + (long)(j - v.lo[1]) * v.jstride + (long)(k - v.lo[2]) * v.kstride;
 }
 
+// The four coefficients of a fit, 32-byte aligned: one 256-bit load, so that a
+// warp reading consecutive fits moves whole lines.  Four 8-byte loads of
+// stride 32 touched every sector four times (2.5 sectors a clock in L1, and
+// long_scoreboard the largest stall).
+struct Fit {
+  double c0, c1, c2, c3;
+};
+__device__ __forceinline__ Fit load_fit(const double* c)
+{
+  Fit f;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(f.c0), "=d"(f.c1), "=d"(f.c2), "=d"(f.c3) : "l"(c));
+  return f;
+}
 __device__ __forceinline__ double fit3(const double* c, double L0, double L1, double L2)
 {
-  return c[0] + c[1] * L0 + c[2] * L1 + c[3] * L2;
+  const Fit f = load_fit(c);
+  return f.c0 + f.c1 * L0 + f.c2 * L1 + f.c3 * L2;
 }
+
+// Resident blocks per SM asked of the compiler: the kernel waits on loads and
+// on the exp's chain, so warps count until the registers they leave spill the
+// exp (heptane, 40,320 cells: 1149 us before the 256-bit loads, 928 at two
+// blocks, 926 at three, 877 at four; dodecane_lu, 32,768 cells: 530, then 422
+// at three and 447 at four; drm19 64^3: 957, then 929 at three, 936 at four).
+__host__ __device__ constexpr int tr_min_blocks(int nb) { return nb == 3 ? 4 : 3; }
 
 // shared memory of a block: Y, D, chi tiles [N][TT]; per warp X, Y [NP]
 // (NP = N, or 32 NB zero-padded) and, with NB == 0, the cell's E matrix
@@ -93,7 +114,7 @@ __host__ __device__ inline size_t tr_smem_doubles(int N, int tt, int nb)
 // TT cells per block tile; NB = 0: the E-matrix form (N <= 32), else the
 // species-block form with NB blocks of 32
 template <int TT, int NB>
-__global__ void __launch_bounds__(TR_THREADS) k_transport(DevMech M, DevTrans t, TrBox b, int flags, long ncells)
+__global__ void __launch_bounds__(TR_THREADS, tr_min_blocks(NB)) k_transport(DevMech M, DevTrans t, TrBox b, int flags, long ncells)
 {
   constexpr int TEAM = 32, TEAMS = TR_WARPS;
   extern __shared__ __align__(16) double trs[];
@@ -245,8 +266,8 @@ __global__ void __launch_bounds__(TR_THREADS) k_transport(DevMech M, DevTrans t,
           a = 0.0;
           for (int jj = tm.lane; jj < N; jj += TEAM) {
             if (jj == i) continue;
-            const double* c = t.fittdrat + 4 * (jj + N * n);
-            a += X[jj] * (c[0] + T * (c[1] + T * (c[2] + T * c[3])));
+            const Fit c = load_fit(t.fittdrat + 4 * (jj + N * n));
+            a += X[jj] * (c.c0 + T * (c.c1 + T * (c.c2 + T * c.c3)));
           }
           const double ch = tm.sum(a);
           if (tm.lane == 0) Ct[(size_t)i * TT + cc] = ch * X[i];
@@ -287,6 +308,7 @@ int upload_transport(const PPBTransTables* t, DeviceTransport* out)
   const int N = t->nsp, L = t->nlite;
   std::vector<double> d;
   auto put = [&](const double* p, size_t n) {
+    while (d.size() % 4) d.push_back(0.0); // fits are loaded 32 bytes at a time
     const size_t o = d.size();
     d.insert(d.end(), p, p + n);
     return o;
