@@ -161,18 +161,17 @@ struct AdjWork {
   double* ybuf; // [n]
   double* tmp;  // [n]
   double* Jc;   // [n * n] df/dy, column-major Jc[j*n + i] = d f_i / d y_j
-  double* AT;   // [n * n] FP64 LU of I - gamma Jc or of its transpose
+  double* AT;   // [n * (n + 1)] FP64 LU of I - gamma Jc or of its transpose, and the row order
   double* jxa;  // [5R] per-reaction factors kf, kr, fac, dq/dT, dq/dlnk
   double* gacc; // [3R] parameter gradient of this warp's cells
   int* piv;     // [n]
-  int* perm;    // [n] row order (scratch of the factorisation)
 };
 
 __host__ __device__ inline size_t adj_bytes(int N, int R)
 {
   const size_t n = N + 1;
-  const size_t d = 6 * n + 10 * n + 1 + 2 * n * n + 6 * (size_t)R + 3 * (size_t)R;
-  return ((d * 8 + 8 * n) + 15) & ~size_t(15);
+  const size_t d = 6 * n + 10 * n + 1 + 2 * n * n + n + 6 * (size_t)R + 3 * (size_t)R;
+  return ((d * 8 + 4 * n) + 15) & ~size_t(15);
 }
 
 
@@ -192,11 +191,10 @@ __device__ inline void carve_adj(AdjWork& a, char* base, int N, int R)
   a.ybuf = p; p += n;
   a.tmp = p; p += n;
   a.Jc = p; p += (size_t)n * n;
-  a.AT = p; p += (size_t)n * n;
+  a.AT = p; p += (size_t)n * (n + 1);
   a.jxa = p; p += 6 * (size_t)R;
   a.gacc = p; p += 3 * (size_t)R;
   a.piv = (int*)p;
-  a.perm = a.piv + n;
 }
 
 // Point at which the right-hand side was differentiated.
@@ -400,7 +398,7 @@ __device__ void jc_mul(const Team<TEAM>& tm, int n, const double* Jc, const doub
 // line, as the solve below: the sweeps keep one copy of each).
 template <int TEAM, int PER>
 __device__ __noinline__ int adj_factor(const Team<TEAM>& tm, int n, const double* Jc, double gamma, bool transpose,
-                                       double* A, int* piv, int* perm)
+                                       double* A, int* piv)
 {
   for (int i = tm.lane; i < n; i += TEAM) {
     for (int j = 0; j < n; j++) {
@@ -411,7 +409,7 @@ __device__ __noinline__ int adj_factor(const Team<TEAM>& tm, int n, const double
     }
   }
   tm.sync();
-  return lu_factor_team<TEAM, double, PER>(tm, A, n, piv, perm);
+  return lu_factor_team<TEAM, double, PER>(tm, A, n, piv);
 }
 
 template <int TEAM>
@@ -609,7 +607,7 @@ struct AdjSweep {
         tangent_rhs(pt, a.lam, dE, dp, a.mu);
         for (int i = tm.lane; i < n; i += TEAM) a.mu[i] = gamma * a.mu[i] - rl1 * a.lam[n + i];
         tm.sync();
-        if (adj_factor<TEAM, PER>(tm, n, a.Jc, gamma, false, a.AT, a.piv, a.perm)) return ST_ADJ_SINGULAR;
+        if (adj_factor<TEAM, PER>(tm, n, a.Jc, gamma, false, a.AT, a.piv)) return ST_ADJ_SINGULAR;
         adj_solve<TEAM>(tm, a.AT, n, a.piv, a.mu);
         for (int i = tm.lane; i < n; i += TEAM) {
           const double d = a.mu[i];
@@ -697,7 +695,7 @@ struct ItemLayout {
 __host__ __device__ inline size_t item_bytes(int N, int R)
 {
   const size_t n = N + 1;
-  return ((8 * (13 * n + 6 * (size_t)R + 2 * n * n) + 8 * n) + 15) & ~size_t(15);
+  return ((8 * (14 * n + 6 * (size_t)R + 2 * n * n) + 4 * n) + 15) & ~size_t(15);
 }
 
 template <int TEAM, int PER>
@@ -723,10 +721,9 @@ __device__ void eval_item(const Team<TEAM>& tm, const DevMech& M, int rtype, dou
   a.fE = p; p += n;
   a.ybuf = p; p += n;
   a.Jc = p; p += (size_t)n * n;
-  a.AT = p; p += (size_t)n * n;
+  a.AT = p; p += (size_t)n * (n + 1);
   a.jxa = p; p += 5 * (size_t)R;
   a.piv = (int*)p;
-  a.perm = a.piv + n;
   for (int i = tm.lane; i < n; i += TEAM) {
     a.ybuf[i] = yg[i];
     w.src[i] = (i < N && srcg) ? srcg[i] : 0.0;
@@ -734,7 +731,7 @@ __device__ void eval_item(const Team<TEAM>& tm, const DevMech& M, int rtype, dou
   tm.sync();
   const AdjPoint pt = rhs_exact_jacobian<TEAM, PER, double>(tm, M, rtype, t, a.ybuf, rhoe, rhoesrc, w.src, w, a);
   int sing = 0;
-  if (gamma != 0.0) sing = adj_factor<TEAM, PER>(tm, n, a.Jc, gamma, true, a.AT, a.piv, a.perm);
+  if (gamma != 0.0) sing = adj_factor<TEAM, PER>(tm, n, a.Jc, gamma, true, a.AT, a.piv);
   for (int i = tm.lane; i < n * n; i += TEAM) item[i] = a.Jc[i];
   if (gamma != 0.0)
     for (int i = tm.lane; i < n * n; i += TEAM) item[IL.at + i] = a.AT[i];

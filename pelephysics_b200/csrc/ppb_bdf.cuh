@@ -375,61 +375,46 @@ __device__ __forceinline__ void pivot_key(float a, unsigned& hi, unsigned& lo)
   lo = 0u;
 }
 
-// x - u l where the pivot row's entry u is nonzero (else x, also against a
-// multiplier that is not finite): a select, no branch.
-template <typename LT>
-__device__ __forceinline__ LT lu_update(LT x, LT u, LT l)
-{
-  const LT v = x - u * l;
-  return u != (LT)0 ? v : x;
-}
-
 // The same factorisation by a team, every entry by the same operations in the
-// same order; perm gets the row order (row i of PA is row perm[i] of A).
+// same order.  A has an (n + 1)-th column that takes part in the row swaps and
+// ends as the row order: row i of PA is row A[n n + i] of A.
 //
-// It is bound by the latency of the chain from one column to the next, so the
-// chain is kept short.  Lane r of a warp holds row k + r (+ 32, + 64) of
-// column k; the largest magnitude is found by integer max reductions over the
-// bits of |a| (one instruction each; two for FP64) and a ballot for the first
-// row holding it, where a butterfly of doubles takes five levels of two
-// shuffles and a compare.  The row swap is part of the update: a lane reads
-// the pivot row's entry and the displaced row's entry of each column it
-// updates and writes both back, so no pass and no barrier of its own.  With
-// 16 rows or fewer left, the lanes split into groups that take several
-// columns at a time.
+// A warp alone runs at about six clocks an instruction here (instruction
+// fetch and dependent latency), so the count of instructions decides.  Lane r
+// holds row k + r (+ 32, + 64) of column k; the largest magnitude is found by
+// integer max reductions over the bits of |a| (one instruction each, two for
+// FP64) and a ballot for the first row holding it.  The rows are swapped in
+// one pass, a column per lane.  With 16 rows or fewer left, the lanes split
+// into groups that update several columns at a time.
+// The update skips the zero entries of the pivot row only where a multiplier
+// is not finite: elsewhere x - 0 l is x.
 // Several warps: every warp finds the pivot by itself (no barrier) and owns
 // the columns j with j mod NW equal to its number, for the swap and the
-// update; column k itself, which every warp reads, is scaled by its owner
-// after the next column's barrier.  One barrier a column.
-// drm19 (22 x 22, one warp alone on its SM): 39,700 SM clocks before.
+// update; column k itself, which every warp reads, is swapped and scaled by
+// its owner after the next column's barrier.  One barrier a column.
 template <int TEAM, typename LT, int RPL>
-__device__ __forceinline__ int lu_factor_team(const Team<TEAM>& tm, LT* A, int n, int* piv, int* perm)
+__device__ __forceinline__ int lu_factor_team(const Team<TEAM>& tm, LT* A, int n, int* piv)
 {
   constexpr int W = Team<TEAM>::W, NW = Team<TEAM>::NW;
   const int wl = tm.lane % W, wid = tm.lane / W;
   const unsigned mask = tm.mask;
-  int pr[RPL]; // the row order: entries wl + W c
+  for (int i = tm.lane; i < n; i += TEAM) A[n * n + i] = (LT)i;
   LT held[RPL]; // the scaled column the warp still has to write (NW > 1)
-  LT held_p = (LT)0;
 #pragma unroll
-  for (int c = 0; c < RPL; c++) {
-    pr[c] = wl + W * c;
-    held[c] = (LT)0;
-  }
+  for (int c = 0; c < RPL; c++) held[c] = (LT)0;
+  tm.sync();
+#pragma unroll 1
   for (int k = 0; k < n; k++) {
     LT* colk = A + k * n;
     if constexpr (NW > 1) {
-      __syncthreads(); // column k is final on every warp
-      if (k > 0 && wid == (k - 1) % NW) {
-        // the owner's scaled column k - 1
-        LT* cp = colk - n;
+      if (k > 0) {
+        __syncthreads(); // column k is final on every warp
+        if (wid == (k - 1) % NW) { // the owner's column k - 1
 #pragma unroll
-        for (int c = 0; c < RPL; c++) {
-          const int i = k - 1 + wl + W * c;
-          if (i > k - 1 && i < n) cp[i] = held[c];
+          for (int c = 0; c < RPL; c++)
+            if (k - 1 + wl + W * c < n) (colk - n)[k - 1 + wl + W * c] = held[c];
+          __syncwarp();
         }
-        if (wl == 0) cp[k - 1] = held_p;
-        __syncwarp();
       }
     }
     // ---- the pivot
@@ -465,116 +450,78 @@ __device__ __forceinline__ int lu_factor_team(const Team<TEAM>& tm, LT* A, int n
         found = true;
       }
     }
-    const LT ak = __shfl_sync(mask, a[0], 0, W); // the displaced row's entry
-    const LT mult = (LT)1.0 / pv;
     if (tm.lane == 0) piv[k] = l;
-    if (l != k) { // row order
-      int pk = 0, pl = 0;
-#pragma unroll
-      for (int c = 0; c < RPL; c++) {
-        if (k / W == c) pk = __shfl_sync(mask, pr[c], k % W, W);
-        if (l / W == c) pl = __shfl_sync(mask, pr[c], l % W, W);
-      }
-#pragma unroll
-      for (int c = 0; c < RPL; c++) {
-        const int i = wl + W * c;
-        if (i == k) pr[c] = pl;
-        if (i == l) pr[c] = pk;
+    // ---- the row swap: column j by lane j (of its owner)
+    const LT ak = __shfl_sync(mask, a[0], 0, W); // the displaced row's entry
+    if (l != k) {
+      for (int j = wid + NW * wl; j <= n; j += NW * W) {
+        if (NW > 1 && j == k) continue; // every warp reads it
+        LT* cj = A + j * n;
+        const LT t = cj[k];
+        cj[k] = cj[l];
+        cj[l] = t;
       }
     }
+    const LT mult = (LT)1.0 / pv;
     // ---- the multipliers of the lane's rows
     LT lik[RPL];
+    bool fin = true;
 #pragma unroll
-    for (int c = 0; c < RPL; c++) lik[c] = (k + wl + W * c == l ? ak : a[c]) * mult;
-    // ---- the factor's earlier columns: the swap alone
-    if (l != k) {
-      for (int j = wid + NW * wl; j < k; j += NW * W) {
-        const LT t = A[j * n + k];
-        A[j * n + k] = A[j * n + l];
-        A[j * n + l] = t;
-      }
+    for (int c = 0; c < RPL; c++) {
+      lik[c] = (k + wl + W * c == l ? ak : a[c]) * mult;
+      fin = fin && (lik[c] - lik[c] == (LT)0);
     }
+    fin = __all_sync(mask, fin);
+    __syncwarp(mask);
     if constexpr (NW == 1) {
 #pragma unroll
       for (int c = 0; c < RPL; c++) {
         const int i = k + wl + W * c;
-        if (i == k) colk[i] = pv;
-        else if (i < n) colk[i] = lik[c];
+        if (i > k && i < n) colk[i] = lik[c];
       }
     } else {
 #pragma unroll
-      for (int c = 0; c < RPL; c++) held[c] = lik[c];
-      held_p = pv;
+      for (int c = 0; c < RPL; c++) held[c] = k + wl + W * c == k ? pv : lik[c];
     }
-    // ---- swap and update of the later columns
+    // ---- the update of the later columns
     if constexpr (NW == 1 && RPL == 1) {
       const int m = n - 1 - k; // rows left
       if (m > 0) {
-        const int s = m > 1 ? 32 - __clz(m - 1) : 0; // 2^s rows (or more) a group
-        const int G = W >> s, r = wl & ((1 << s) - 1), g = wl >> s;
-        const int i = k + 1 + r;
+        const int s = m > 1 ? 32 - __clz(m - 1) : 0; // groups of 2^s >= m lanes
+        const int r = wl & ((1 << s) - 1), g = wl >> s;
         const LT lr = __shfl_sync(mask, lik[0], (1 + r) % W, W);
-        constexpr int U = 4;
-        for (int jb = k + 1; jb < n; jb += U * G) {
-          LT t[U], u[U], x[U];
-#pragma unroll
-          for (int q = 0; q < U; q++) {
-            const int j = jb + q * G + g;
-            const LT* cj = A + (j < n ? j : k) * n;
-            t[q] = cj[k];
-            u[q] = cj[l];
-            x[q] = cj[r < m ? i : k];
-          }
-          __syncwarp(mask);
-#pragma unroll
-          for (int q = 0; q < U; q++) {
-            const int j = jb + q * G + g;
-            LT* cj = A + j * n;
-            if (j < n && r < m) cj[i] = lu_update(i == l ? t[q] : x[q], u[q], lr);
-            if (j < n && r == 0) cj[k] = u[q];
+        const int step = (W >> s) * n;
+        const LT* pu = A + (k + 1 + g) * n + k; // the pivot row's entry
+        const int end = n * n;
+        int at = (k + 1 + g) * n + k;
+        if (r < m) {
+          if (fin) {
+#pragma unroll 2
+            for (; at < end; at += step, pu += step) const_cast<LT*>(pu)[1 + r] -= pu[0] * lr;
+          } else {
+            for (; at < end; at += step, pu += step)
+              if (pu[0] != (LT)0) const_cast<LT*>(pu)[1 + r] -= pu[0] * lr;
           }
         }
       }
       __syncwarp(mask);
     } else {
-      constexpr int U = 2;
-      // first column after k that the warp owns
-      int j0 = k + 1;
-      if constexpr (NW > 1) j0 += ((wid - j0) % NW + NW) % NW;
-      for (int jb = j0; jb < n; jb += U * NW) {
-        LT t[U], u[U], x[U][RPL];
-#pragma unroll
-        for (int q = 0; q < U; q++) {
-          const int j = jb + q * NW;
-          const LT* cj = A + (j < n ? j : jb) * n;
-          t[q] = cj[k];
-          u[q] = cj[l];
+      int j = k + 1; // the first column after k that the warp owns
+      if constexpr (NW > 1) j += ((wid - j) % NW + NW) % NW;
+#pragma unroll 2
+      for (; j < n; j += NW) {
+        LT* cj = A + j * n;
+        const LT u = cj[k];
+        if (fin || u != (LT)0) {
 #pragma unroll
           for (int c = 0; c < RPL; c++) {
             const int i = k + wl + W * c;
-            x[q][c] = i < n ? cj[i] : (LT)0;
-          }
-        }
-        __syncwarp(mask);
-#pragma unroll
-        for (int q = 0; q < U; q++) {
-          const int j = jb + q * NW;
-          LT* cj = A + j * n;
-#pragma unroll
-          for (int c = 0; c < RPL; c++) {
-            const int i = k + wl + W * c;
-            const LT v = lu_update(i == l ? t[q] : x[q][c], u[q], lik[c]);
-            if (j < n && i < n) cj[i] = i == k ? u[q] : v;
+            if (i > k && i < n) cj[i] -= u * lik[c];
           }
         }
       }
       __syncwarp(mask);
     }
-  }
-  if (wid == 0) {
-#pragma unroll
-    for (int c = 0; c < RPL; c++)
-      if (wl + W * c < n) perm[wl + W * c] = pr[c];
   }
   tm.sync();
   return 0;
@@ -718,28 +665,29 @@ __device__ __forceinline__ void lu_solve_reg(const Team<TEAM>& tm, const LT* A, 
         }
       }
     }
+    // an entry's quotient is formed by its own lane, with its diagonal entry
+    // and reciprocal in registers, and then broadcast
 #pragma unroll
     for (int kb = RPL - 1; kb >= 0; kb--) {
       const int k1 = kb < RPL - 1 ? W : NN - W * kb;
-#pragma unroll 3
+      const int d = wl + W * kb < NN ? wl + W * kb : 0;
+      const double add = (double)A[d * NN + d], yd = dinv[d];
+      double num = 0.0; // the lane's numerator
+#pragma unroll 2
       for (int kk = k1 - 1; kk >= 0; kk--) {
         const int k = W * kb + kk;
-        const double b0 = __shfl_sync(tm.mask, x[kb], kk, W);
-        const double bk = quotient(b0, (double)A[k * NN + k], dinv[k]);
-        // |b| within 2^-500 .. 2^500, or zero
-        const unsigned e = ((unsigned)__double2hiint(b0) >> 20) & 0x7ffu;
-        bad = bad || (e - 523u > 1000u && b0 != 0.0);
+        const double own = quotient(x[kb], add, yd);
+        const double bk = __shfl_sync(tm.mask, own, kk, W);
 #pragma unroll
-        for (int c = 0; c <= kb; c++) {
-          const int i = wl + W * c;
-          const double a = (double)A[k * NN + (i < NN ? i : 0)];
-          if (i == k) {
-            x[c] = bk;
-          } else if (i < k) {
-            x[c] -= a * bk;
-          }
-        }
+        for (int c = 0; c < kb; c++) x[c] -= (double)A[k * NN + wl + W * c] * bk;
+        const double a = (double)A[k * NN + d];
+        if (wl == kk) num = x[kb];
+        if (wl == kk) x[kb] = own;
+        if (wl < kk) x[kb] -= a * bk;
       }
+      // |numerator| within 2^-500 .. 2^500, or zero
+      const unsigned e = ((unsigned)__double2hiint(num) >> 20) & 0x7ffu;
+      bad = bad || (e - 523u > 1000u && num != 0.0);
     }
   }
   if constexpr (NW > 1) {
@@ -1095,8 +1043,11 @@ struct Bdf {
     tm.sync();
     int ier;
     if constexpr (TEAM > 1) {
-      ier = lu_factor_team<TEAM, LT, (n + Team<TEAM>::W - 1) / Team<TEAM>::W>(tm, w.A, n, w.piv, w.perm) ? 1 : 0;
-      if (!ier) diag_recip(tm, w.A, w.dinv, n);
+      ier = lu_factor_team<TEAM, LT, (n + Team<TEAM>::W - 1) / Team<TEAM>::W>(tm, w.A, n, w.piv) ? 1 : 0;
+      if (!ier) {
+        for (int i = tm.lane; i < n; i += TEAM) w.perm[i] = (int)w.A[n * n + i];
+        diag_recip(tm, w.A, w.dinv, n);
+      }
     } else {
       ier = lu_factor<LT>(w.A, n, w.piv) ? 1 : 0;
     }

@@ -23,7 +23,7 @@ template <typename LT>
 __host__ __device__ inline size_t a_region_bytes(int N, int R)
 {
   const size_t n = N + 1;
-  size_t a = n * n * sizeof(LT);
+  size_t a = n * (n + 1) * sizeof(LT); // the row order is a column of the factor
   const size_t jx = 40 * (size_t)R;
   if (sizeof(LT) == sizeof(double) && jx > a) a = jx;
   return (a + 15) & ~size_t(15);
