@@ -272,7 +272,7 @@ int ppb_transport_box(const char* mechanism, int use_soret, const int lo[3], con
  * reference).  For callers that must not have a library allocate GPU memory,
  * e.g. applications whose device memory is owned by an arena allocator
  * (AMReX-based codes hand every device buffer out of the AMReX Arena).  It
- * runs the tuned engine out of one static device array of 32 MiB per GPU
+ * runs the tuned engine out of one static device array of 34 MiB per GPU
  * holding the mechanism tables and the per-call scratch, and calls no
  * cudaMalloc/cudaFree.  Limits: at most
  * floor((30 MiB - 1 KiB) / (8 (2N+1) + 12)) cells per call (drm19: 88,360;

@@ -345,6 +345,40 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
   }
   pk.put(off_joff + N * sizeof(int), &k, 1);
   pk.used = off_jc + jtotal * sizeof(double);
+  {
+    int jl = 0;
+    for (int sp = 0; sp < N; sp++) {
+      int c = 0;
+      for (int r = 0; r < R; r++)
+        for (int j = 0; j < t->rx_jn_n[r]; j++)
+          c += (t->rx_jn_sp[r * PPB_MAXJN + j] == sp && t->rx_jn_c[r * PPB_MAXJN + j] != 0.0);
+      jl = c > jl ? c : jl;
+    }
+    const size_t off_n = (pk.used + 15) & ~size_t(15);
+    const size_t off_e = (off_n + N * sizeof(int) + 15) & ~size_t(15);
+    for (int sp = 0; sp < N; sp++) {
+      int c = 0;
+      for (int r = 0; r < R; r++)
+        for (int j = 0; j < t->rx_jn_n[r]; j++) {
+          const double nu = t->rx_jn_c[r * PPB_MAXJN + j];
+          if (t->rx_jn_sp[r * PPB_MAXJN + j] != sp || nu == 0.0) continue;
+          unsigned long long bits;
+          memcpy(&bits, &nu, 8);
+          if (bits << 16) pk.overflow = true;
+          const unsigned e = (unsigned)(bits >> 48) << 16 | (unsigned)r;
+          pk.put(off_e + ((size_t)c * N + sp) * sizeof(unsigned), &e, 1);
+          c++;
+        }
+      pk.put(off_n + sp * sizeof(int), &c, 1);
+      for (; c < jl; c++) {
+        const unsigned e = 0;
+        pk.put(off_e + ((size_t)c * N + sp) * sizeof(unsigned), &e, 1);
+      }
+    }
+    pk.used = off_e + (size_t)jl * N * sizeof(unsigned);
+    set_off(dm.jh_n, off_n);
+    set_off(dm.jh, off_e);
+  }
   set_off(dm.jg_off, off_joff);
   set_off(dm.jg_rx, off_jrx);
   set_off(dm.jg_c, off_jc);
@@ -488,26 +522,87 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
           if (t->rx_rps_sp[r * PPB_MAXPS + j] == k) return true;
       return false;
     };
-    int tot = 0;
-    for (int k = 0; k < N; k++)
-      for (int r = 0; r < R; r++) tot += reaches(r, k);
-    const size_t off_jcoff = (pk.used + 15) & ~size_t(15);
-    const size_t off_jcrx = (off_jcoff + (N + 1) * sizeof(int) + 15) & ~size_t(15);
+    int jcl = 0;
+    for (int k = 0; k < N; k++) {
+      int c = 0;
+      for (int r = 0; r < R; r++) c += reaches(r, k);
+      jcl = c > jcl ? c : jcl;
+    }
+    jcl++; // an entry of padding ends every list
+    const size_t off_jcn = (pk.used + 15) & ~size_t(15);
+    const size_t off_jc = (off_jcn + N * sizeof(int) + 15) & ~size_t(15);
+    // derivative of a phase space by species k: its multiplicity and the other
+    // factors in species order
+    auto deriv = [&](const int* sp, const double* c, int ns, int k, unsigned char (&f)[2]) {
+      int mult = 0, q = 0;
+      for (int j = 0; j < ns; j++) {
+        int o = (int)c[j];
+        if (sp[j] == k) {
+          mult = o;
+          o--;
+        }
+        for (; o > 0; o--)
+          if (q < 2) f[q++] = (unsigned char)sp[j];
+          else pk.overflow = true;
+      }
+      if (mult > 15) pk.overflow = true;
+      return mult;
+    };
     int e = 0;
     for (int k = 0; k < N; k++) {
-      pk.put(off_jcoff + k * sizeof(int), &e, 1);
+      e = 0;
       for (int r = 0; r < R; r++) {
         if (!reaches(r, k)) continue;
-        const unsigned short rr = (unsigned short)r;
-        pk.put(off_jcrx + e * sizeof(unsigned short), &rr, 1);
+        JcEntry je;
+        memset(&je, 0, sizeof(je));
+        je.r = (unsigned short)r;
+        for (int q = 0; q < 2; q++) je.fs[q] = je.rs[q] = (unsigned char)N;
+        const int kind = t->rx_kind[r];
+        int mf = 0, mr = 0;
+        for (int j = 0; j < t->rx_fps_n[r]; j++)
+          if (t->rx_fps_sp[r * PPB_MAXPS + j] == k) mf = 1;
+        if (t->rx_rev[r])
+          for (int j = 0; j < t->rx_rps_n[r]; j++)
+            if (t->rx_rps_sp[r * PPB_MAXPS + j] == k) mr = 1;
+        if (mf) mf = deriv(t->rx_fps_sp + r * PPB_MAXPS, t->rx_fps_c + r * PPB_MAXPS, t->rx_fps_n[r], k, je.fs);
+        if (mr) mr = deriv(t->rx_rps_sp + r * PPB_MAXPS, t->rx_rps_c + r * PPB_MAXPS, t->rx_rps_n[r], k, je.rs);
+        je.c = (unsigned char)(mf | (mr << 4));
+        je.flags = (unsigned char)((mf ? JC_INR : 0) | (mr ? JC_INP : 0));
+        je.e = 1.0;
+        if (kind == PPB_RX_THIRD || kind == PPB_RX_TROE || kind == PPB_RX_LINDEMANN) {
+          je.flags |= JC_ALPHA;
+          for (int q = t->eff_off[r]; q < t->eff_off[r + 1]; q++)
+            if (t->eff_sp[q] == k) {
+              je.e = t->eff_e[q];
+              je.flags |= JC_LISTED;
+            }
+        }
+        int m = 0;
+        for (int j = 0; j < t->rx_jn_n[r]; j++) {
+          if (t->rx_jn_c[r * PPB_MAXJN + j] == 0.0) continue;
+          unsigned long long bits;
+          memcpy(&bits, &t->rx_jn_c[r * PPB_MAXJN + j], 8);
+          if (m >= 5 || (bits << 16)) {
+            pk.overflow = true;
+            break;
+          }
+          je.nu[m] = (unsigned short)(bits >> 48);
+          je.sp[m++] = (unsigned char)t->rx_jn_sp[r * PPB_MAXJN + j];
+        }
+        for (int w = 0; w < 2; w++)
+          pk.put(off_jc + ((size_t)(2 * e + w) * N + k) * 16, reinterpret_cast<const char*>(&je) + 16 * w, 16);
         e++;
       }
+      pk.put(off_jcn + k * sizeof(int), &e, 1);
+      for (; e < jcl; e++) {
+        const char z[16] = {};
+        for (int w = 0; w < 2; w++) pk.put(off_jc + ((size_t)(2 * e + w) * N + k) * 16, z, 16);
+      }
     }
-    pk.put(off_jcoff + N * sizeof(int), &e, 1);
     if (R > 65535) pk.overflow = true;
-    pk.used = off_jcrx + (size_t)tot * sizeof(unsigned short);
-    set_off(dm.jc_off, off_jcoff);
-    set_off(dm.jc_rx, off_jcrx);
+    pk.used = off_jc + (size_t)2 * jcl * N * 16;
+    set_off(dm.jc_n, off_jcn);
+    set_off(dm.jc, off_jc);
     // member lists (phase-space species only) and the third-body list
     auto member = [&](int r, int k) {
       for (int j = 0; j < t->rx_fps_n[r]; j++)

@@ -87,11 +87,12 @@ struct DevMech {
   const struct FoPack* fop;
   const unsigned* effmask; // 4 words per reaction: species with a listed efficiency
   const double* effd;      // [third-body reactions][nsp] efficiencies, 1 where unlisted
-  // per species k, in reaction order, the reactions whose Jacobian row
-  // d q_r / d c_k can be nonzero: every third-body / fall-off reaction and
-  // the reactions with k in their forward or (reversible) reverse phase space
-  const int* jc_off;
-  const unsigned short* jc_rx;
+  // the Jacobian's columns: for species k, in reaction order, the reactions
+  // whose d q_r / d c_k can be nonzero (every third-body / fall-off reaction
+  // and the reactions with k in their forward or, reversible, reverse phase
+  // space): word w of entry j < jc_n[k] at jc[(2 j + w) nsp + k] (JcEntry)
+  const int* jc_n;
+  const int4* jc;
   // per species k, in reaction order, the reactions with k in their forward
   // or (reversible) reverse phase space; and the third-body / fall-off
   // reactions (al_off = {0, count})
@@ -102,6 +103,9 @@ struct DevMech {
   // species-major gather of the aJacobian net stoichiometry (jn lists)
   const int *jg_off, *jg_rx;
   const double* jg_c;
+  // the same, coalesced (as wg): entry j < jh_n[s] of species s at jh[j nsp + s]
+  const int* jh_n;
+  const unsigned* jh;
   // SRK equation of state: [sqrt(1/Tc) | sqrt(a*) | B | F(omega)], N each
   const double* srk;
   // QSS balance (PPBMechTables: q_rx, q_off, q_term, q_role, q_coef,
@@ -151,6 +155,23 @@ struct alignas(16) RxRate {
 };
 static_assert(sizeof(RxRate) == 48, "RxRate is three 16-byte words");
 enum { RR_REV = 1, RR_ALPHA = 2, RR_RMF = 4, RR_KCPOW = 3 };
+
+// One reaction in one column of the Jacobian, in 32 bytes: the derivative of a
+// phase space is c * sc[s0] * sc[s1] (the factors in species order, the unit
+// slot where there are fewer), the net stoichiometry five species with the top
+// 16 bits of their coefficients as doubles (0: none).
+struct alignas(16) JcEntry {
+  unsigned short r;
+  unsigned char flags;     // JC_INR, JC_INP, JC_ALPHA, JC_LISTED
+  unsigned char c;         // multiplicities: forward, reverse << 4
+  unsigned char fs[2], rs[2];
+  double e;                // third-body efficiency of the column's species
+  unsigned short nu[5];
+  unsigned char sp[5], pad;
+};
+static_assert(sizeof(JcEntry) == 32, "JcEntry is two 16-byte words");
+enum { JC_INR = 1, JC_INP = 2, JC_ALPHA = 4, JC_LISTED = 8 };
+
 constexpr int WG_UNROLL = 8;  // gather entries loaded together
 constexpr int EFF_UNROLL = 4; // efficiencies loaded together
 
@@ -1330,10 +1351,12 @@ __device__ void ajacobian_packed(
   // (2) wdot and the d/dT row, reaction order per species
   for (int s = tm.lane; s < N; s += TEAM) {
     double w = 0.0, d = 0.0;
-    const int g1 = __ldg(M.jg_off + s + 1);
-    for (int gi = __ldg(M.jg_off + s); gi < g1; gi++) {
-      const int r = __ldg(M.jg_rx + gi);
-      const double nu = __ldg(M.jg_c + gi);
+    const int cnt = __ldg(M.jh_n + s);
+#pragma unroll 4
+    for (int j = 0; j < cnt; j++) {
+      const unsigned e = __ldg(M.jh + j * N + s);
+      const double nu = __hiloint2double((int)(e & 0xffff0000u), 0);
+      const int r = (int)(e & 0xffffu);
       w += nu * rs.qd[r];
       d += nu * jx[4 * r + 3];
     }
@@ -1344,74 +1367,49 @@ __device__ void ajacobian_packed(
   // reactions that reach its column in reaction order (the per-entry
   // accumulation order of the generated code; dq carries the last dq/dc_k of
   // a third-body reaction, which the consP == 0 form reuses for a
-  // zero-efficiency species without a rate term)
+  // zero-efficiency species without a rate term).  The entries hold what the
+  // walk needs of a reaction, one coalesced load ahead; from the reactions'
+  // 80-byte records, with their slot lists searched for k, a column of drm19
+  // took 2,000 instructions more than its arithmetic.
 #pragma unroll
   for (int qq = 0; qq < PER; qq++) {
     const int k = tm.lane + qq * TEAM;
     if (k >= N) break;
     double dq = 0.0;
     double* Jk = J + k * n;
-    const unsigned word_i = (unsigned)(k >> 5), bit = 1u << (k & 31);
-    const int e1 = __ldg(M.jc_off + k + 1);
-    for (int ei = __ldg(M.jc_off + k); ei < e1; ei++) {
-      const int r = __ldg(M.jc_rx + ei);
-      const RxPack p = load_rx(M, r);
-      const bool falloff = (p.fo != 255);
-      const bool has_alpha = (p.kind == PPB_RX_THIRD) || falloff;
-      const bool rev = p.rev != 0;
-      const double k_f = jx[4 * r + 0];
-      const double k_r = jx[4 * r + 1];
-      const double fac = jx[4 * r + 2];
-      const bool inr = slots_has(p.fsp, k);
-      const bool inp = rev && slots_has(p.rsp, k);
+    const int cnt = __ldg(M.jc_n + k);
+    const int4* pe = M.jc + k;
+    int4 w0 = __ldg(pe), w1 = __ldg(pe + N);
+#pragma unroll 1
+    for (int j = 0; j < cnt; j++) {
+      JcEntry p;
+      reinterpret_cast<int4*>(&p)[0] = w0;
+      reinterpret_cast<int4*>(&p)[1] = w1;
+      pe += 2 * N; // the next entry (the list ends with one of padding)
+      w0 = __ldg(pe);
+      w1 = __ldg(pe + N);
+      const double* jr = jx + 4 * p.r;
+      const double fac = jr[2];
+      const double pf = ((double)(p.c & 15) * sc[p.fs[0]]) * sc[p.fs[1]];
+      const double pr = ((double)(p.c >> 4) * sc[p.rs[0]]) * sc[p.rs[1]];
+      const bool inr = (p.flags & JC_INR) != 0, inp = (p.flags & JC_INP) != 0, alpha = (p.flags & JC_ALPHA) != 0;
       double d = 0.0;
-      bool apply = false;
-      if (has_alpha) {
-        const bool listed = (__ldg(M.effmask + 4 * r + word_i) & bit) != 0u;
-        const double* ed = M.effd + (size_t)p.aslot * N;
-        if (consP == 1) {
-          if (listed) {
-            d = (__ldg(ed + k) - 1) * fac;
-            apply = true;
-          }
-          if (inr) {
-            d += k_f * slots_dproduct(p.fsp, sc, k);
-            apply = true;
-          }
-          if (inp) {
-            d -= k_r * slots_dproduct(p.rsp, sc, k);
-            apply = true;
-          }
-        } else {
-          const double e = listed ? __ldg(ed + k) : 1.0;
-          if (!(e == 0.0 && !inr && !inp)) {
-            if (e == 0.0) {
-              d = 0.0;
-              if (inr) d = k_f * slots_dproduct(p.fsp, sc, k);
-              if (inp) d = (inr ? d : 0.0) - k_r * slots_dproduct(p.rsp, sc, k);
-            } else {
-              d = (e == 1.0) ? fac : e * fac;
-              if (inr) d += k_f * slots_dproduct(p.fsp, sc, k);
-              if (inp) d -= k_r * slots_dproduct(p.rsp, sc, k);
-            }
-            dq = d;
-          }
-          d = dq;
-          apply = true;
-        }
-      } else {
-        if (inr) d += k_f * slots_dproduct(p.fsp, sc, k);
-        if (inp) d -= k_r * slots_dproduct(p.rsp, sc, k);
-        apply = inr || inp;
+      if (alpha) {
+        const double e = consP == 1 ? p.e - 1 : p.e;
+        if (consP == 1 ? (p.flags & JC_LISTED) != 0 : e != 0.0) d = e * fac;
       }
-      if (apply) {
-        #pragma unroll
-        for (int j = 0; j < 6; j++) { // static slot index: the record stays in registers
-          if (j >= p.njn) break;
-          const double nu = (double)p.jnc[j];
-          if (nu != 0) Jk[p.jns[j]] += nu * d;
-        }
+      if (inr) d = __fma_rn(jr[0], pf, d);
+      if (inp) d = __fma_rn(-jr[1], pr, d);
+      if (alpha && consP != 1) {
+        if (p.e == 0.0 && !inr && !inp) d = dq;
+        dq = d;
       }
+      double v[5];
+#pragma unroll
+      for (int q = 0; q < 5; q++) v[q] = Jk[p.sp[q]];
+#pragma unroll
+      for (int q = 0; q < 5; q++)
+        if (p.nu[q]) Jk[p.sp[q]] = __fma_rn(__hiloint2double((int)((unsigned)p.nu[q] << 16), 0), d, v[q]);
     }
   }
   tm.sync();

@@ -7,7 +7,7 @@
 // size and out-of-memory handling assume nobody else calls cudaMalloc), and
 // codes that run next to them in the same process with the memory budget
 // already spent.  For them this entry point works entirely out of one
-// file-scope device array, PPB_NOALLOC_BYTES (32 MiB) per GPU, which holds
+// file-scope device array, PPB_NOALLOC_BYTES (34 MiB) per GPU, which holds
 // the mechanism tables and the per-call scratch (species-major copies of the
 // state and sources, per-cell flags and costs, the work-queue counter and a
 // failure counter).  The array is part of the library image: every GPU that
@@ -35,8 +35,8 @@
 
 namespace ppb {
 enum : size_t {
-  PPB_NOALLOC_BYTES = size_t(32) << 20,  // whole array
-  PPB_NOALLOC_TABLES = size_t(2) << 20,  // mechanism tables region
+  PPB_NOALLOC_BYTES = size_t(34) << 20,  // whole array
+  PPB_NOALLOC_TABLES = size_t(4) << 20,  // mechanism tables region
   PPB_NOALLOC_MAX_DEVICES = 64,
   PPB_NOALLOC_MAX_MECHS = 8,
 };
