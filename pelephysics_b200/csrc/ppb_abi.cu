@@ -442,7 +442,7 @@ static LaunchConfig launch_config(const ppb_reactor* r)
   }
   if (r->opt.warps_per_block > 0) {
     lc.warps_per_block = r->opt.warps_per_block;
-    lc.team = (r->opt.team_lanes == 16 || r->opt.team_lanes == 64 || r->opt.team_lanes == 128) ? r->opt.team_lanes : 32;
+    lc.team = fixed_team(r->t->nsp, r->method, r->opt.warps_per_block, r->opt.team_lanes);
     lc.minb = r->opt.register_budget == 1 ? 1 : 2;
     if (lc.team > 32) { // one cell per block of team / 32 warps, <= 255 registers
       lc.warps_per_block = lc.team / 32;
@@ -477,8 +477,8 @@ static int autotune(ppb_reactor* r, const Batch& b, double dt, cudaStream_t st)
   const int N = r->t->nsp, n = N + 1;
   std::vector<LaunchConfig> cand;
   int max_res = 0;
-  const int big = N <= 21 ? 0 : N <= 64 ? 64 : 128;
-  for (int team : {32, 16, big}) {
+  const int big = species_team(N);
+  for (int team : {32, 16, big, 2 * big}) {
     if (team == 0 || (team == 16 && N > 21)) continue;
     for (int minb : {2, 1}) {
       if (minb == 1 && (r->method != METHOD_BDF || r->opt.lu_fp32) && team <= 32) continue;
@@ -1386,7 +1386,7 @@ int ppb_get_launch_config(ppb_reactor* r, int* warps_per_block, int* team_lanes,
   LaunchConfig tl;
   if (r->opt.warps_per_block <= 0) tuned_config(r, &tl, &ms);
   if (warps_per_block) *warps_per_block = lc.warps_per_block;
-  if (team_lanes) *team_lanes = lc.team;
+  if (team_lanes) *team_lanes = (lc.team > 32 && lc.team == 2 * species_team(r->t->nsp)) ? lc.team / 2 : lc.team;
   if (register_budget) *register_budget = lc.minb;
   if (tuned_ms) *tuned_ms = ms;
   return 0;

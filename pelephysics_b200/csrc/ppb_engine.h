@@ -51,13 +51,25 @@ struct LaunchConfig {
   int warps_per_block = 4;
   int lu_fp32 = 0;
   int persistent = 1; // work queue
-  int team = 32;      // lanes per cell: 32; 16 for <= 21 species; 64 (33..64 species) or 128 (65..128): one
-                      // multi-warp team per block
+  int team = 32;      // lanes per cell: 32; 16 for <= 21 species; 64 (33..64 species) or 128 (65..128), or
+                      // twice that (BDF): one multi-warp team per block
   int minb = 2;       // register budget: >= minb blocks of 256 threads per SM
   int rhsv = 0;       // right-hand side: 0 ideal gas, 1 the SRK e-reactor, 2 a QSS mechanism (the last two:
                       // warp teams, <= 128 registers, difference-quotient Jacobian)
   int rv = -1;        // rendezvous bound the autotuner picked, used when the option is -1 (-1: by block size)
 };
+// Lanes of the multi-warp team with one lane per species (0: none).
+inline int species_team(int nsp) { return nsp <= 21 ? 0 : nsp <= 64 ? 64 : 128; }
+// Lanes of a fixed launch (options warps_per_block = w, team_lanes = lanes):
+// lanes, or twice as many when w asks for twice lanes / 32 warps.  A team the
+// mechanism has not is refused at the launch (1024 lanes: no such kernel).
+inline int fixed_team(int nsp, int method, int w, int lanes)
+{
+  if (lanes == 16) return 16;
+  if (lanes != 64 && lanes != 128) return 32;
+  if (lanes != species_team(nsp)) return 1024;
+  return (method == METHOD_BDF && w == lanes / 16) ? 2 * lanes : lanes;
+}
 // Resident cells per SM of the tuned kernel in configuration lc (0: the
 // configuration does not fit or is not compiled).
 int react_occupancy(const DeviceMechanism& m, int method, const LaunchConfig& lc);

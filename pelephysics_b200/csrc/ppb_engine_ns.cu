@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_react_team(const __grid_constant
 {
   extern __shared__ __align__(16) char smem[];
   if constexpr (TEAM > 32) {
-    __shared__ double red[16];
+    __shared__ double red[4 * (TEAM / 32)];
     __shared__ BdfArrays warp_arrays[TEAM / 32];
     const Team<TEAM> tm(red);
     react_team_body<NS, LT, METHOD, TEAM>(tm, M, o, b, dt, queue, cell_bytes, persistent, smem, warp_arrays);
@@ -189,6 +189,7 @@ typedef void (*TeamKernel)(DevMech, Options, Batch, double, int*, size_t, int);
 
 // Lanes per cell of the multi-warp team compiled for a mechanism: one lane
 // per species (64 for 33..64 species, 128 for 65..128), 0 for <= 21 species.
+// The BDF kernels are compiled with twice as many as well.
 template <int NS>
 constexpr int big_team()
 {
@@ -269,10 +270,17 @@ static TeamKernel team_kernel_part(int method, bool fp32, int team, int minb, in
     if (team > 32) {
       if constexpr (big_team<NS>() > 0 && P == 2) {
         constexpr int BT = big_team<NS>();
-        if (team != BT) return nullptr;
-        if (method == METHOD_RK64) return (TeamKernel)k_react_team<NS, double, METHOD_RK64, BT, 1>;
-        if (fp32) return (TeamKernel)k_react_team<NS, float, METHOD_BDF, BT, 1>;
-        return (TeamKernel)k_react_team<NS, double, METHOD_BDF, BT, 1>;
+        if (team == BT) {
+          if (method == METHOD_RK64) return (TeamKernel)k_react_team<NS, double, METHOD_RK64, BT, 1>;
+          if (fp32) return (TeamKernel)k_react_team<NS, float, METHOD_BDF, BT, 1>;
+          return (TeamKernel)k_react_team<NS, double, METHOD_BDF, BT, 1>;
+        }
+        // twice the lanes: the cell's workspace leaves room for two or three
+        // cells an SM, so that more warps per cell are the only warps to add
+        if (team == 2 * BT && method == METHOD_BDF)
+          return fp32 ? (TeamKernel)k_react_team<NS, float, METHOD_BDF, 2 * BT, 1>
+                      : (TeamKernel)k_react_team<NS, double, METHOD_BDF, 2 * BT, 1>;
+        return nullptr;
       }
       return nullptr;
     }
@@ -345,7 +353,7 @@ static int launch_react_ns(const DeviceMechanism& m, const Options& o, int metho
     return (int)cudaGetLastError();
   }
   const bool fp32 = lc.lu_fp32 && method == METHOD_BDF;
-  const int team = (lc.team == 16 || lc.team > 32) ? lc.team : 32;
+  const int team = lc.team;
   // a multi-warp team is one block
   const int wpb = team > 32 ? team / 32 : (lc.warps_per_block > 0 ? lc.warps_per_block : 4);
   TeamKernel kern = team_kernel<NS>(method, fp32, team, lc.minb, lc.rhsv, wpb);
@@ -383,7 +391,7 @@ template <int NS>
 static int occupancy_ns(const DevMech& M, int method, const LaunchConfig& lc)
 {
   const bool fp32 = lc.lu_fp32 && method == METHOD_BDF;
-  const int team = (lc.team == 16 || lc.team > 32) ? lc.team : 32;
+  const int team = lc.team;
   const int wpb = team > 32 ? team / 32 : (lc.warps_per_block > 0 ? lc.warps_per_block : 4);
   TeamKernel kern = team_kernel<NS>(method, fp32, team, lc.minb, lc.rhsv, wpb);
   if (!kern) return 0;

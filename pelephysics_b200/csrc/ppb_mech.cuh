@@ -190,7 +190,7 @@ static_assert(sizeof(FoPack) == 112, "FoPack is seven 16-byte words");
 // warps, one team per block: warp shuffles, then the warps' partial results
 // through a small shared scratch and __syncthreads).  Every reduction returns
 // the same bits on every lane (fixed combination order).
-// The block-shared scratch of a multi-warp team (2 * warps doubles); warp
+// The block-shared scratch of a multi-warp team (4 * warps doubles); warp
 // teams carry none.
 template <int TEAM, bool MULTI = (TEAM > 32)>
 struct TeamScratch {
@@ -337,16 +337,6 @@ struct Team : TeamScratch<TEAM> {
       return reduce(x, [](double a, double b) { return fmax(a, b); });
     }
   }
-  __device__ __forceinline__ int imax(int x) const
-  {
-    if constexpr (TEAM <= 32) {
-#pragma unroll
-      for (int o = TEAM / 2; o > 0; o >>= 1) x = ::max(x, __shfl_xor_sync(mask, x, o, TEAM));
-      return x;
-    } else {
-      return reduce(x, [](int a, int b) { return ::max(a, b); });
-    }
-  }
   // broadcast from team lane src
   __device__ __forceinline__ double bcast(double x, int src) const
   {
@@ -375,39 +365,6 @@ struct Team : TeamScratch<TEAM> {
       const int v = r[0];
       __syncthreads();
       return v;
-    }
-  }
-  // largest best over the team, ties to the smallest index bi
-  __device__ __forceinline__ void argmax(double& best, int& bi) const
-  {
-    if constexpr (TEAM > 1) {
-#pragma unroll
-      for (int o = W / 2; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(mask, best, o, W);
-        const int oi = __shfl_xor_sync(mask, bi, o, W);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-    }
-    if constexpr (TEAM > 32) {
-      int* ri = reinterpret_cast<int*>(this->red + NW);
-      if ((lane & 31) == 0) {
-        this->red[lane >> 5] = best;
-        ri[lane >> 5] = bi;
-      }
-      __syncthreads();
-      best = this->red[0];
-      bi = ri[0];
-#pragma unroll
-      for (int i = 1; i < NW; i++) {
-        if (this->red[i] > best || (this->red[i] == best && ri[i] < bi)) {
-          best = this->red[i];
-          bi = ri[i];
-        }
-      }
-      __syncthreads();
     }
   }
 };

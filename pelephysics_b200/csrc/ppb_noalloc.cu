@@ -219,7 +219,7 @@ extern "C" int ppb_react_flat_device_noalloc(const char* mechanism, const char* 
   lc.persistent = 1;
   lc.rhsv = o.eos == PPB_EOS_SRK ? 1 : 0;
   lc.warps_per_block = o.warps_per_block;
-  lc.team = (o.team_lanes == 16 || o.team_lanes == 64 || o.team_lanes == 128) ? o.team_lanes : 32;
+  lc.team = fixed_team(t->nsp, method, o.warps_per_block, o.team_lanes);
   lc.minb = o.register_budget == 1 ? 1 : 2;
   if (lc.team > 32) { // one cell per block of team / 32 warps, <= 255 registers
     lc.warps_per_block = lc.team / 32;
