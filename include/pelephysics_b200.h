@@ -66,8 +66,8 @@ typedef struct ppb_options {
   int adjoint_checkpoint_interval; /* accepted BDF steps between adjoint checkpoints, 16 */
   int adjoint_memory_mb;    /* device memory for adjoint checkpoints, tapes and points, 16384 */
   int team_lanes;           /* with warps_per_block > 0: lanes per cell, 32, 16 (<= 21 species), 64
-                               (33..64 species) or 128 (65..128 species); one cell per block. With warps_per_block twice team_lanes / 32 the BDF
-                               runs twice as many lanes a cell (heptane_lu_88sk, FP64 LU: 48k -> 57k cells/s) */
+                               (33..64 species) or 128 (65..128 species; one cell per block; with warps_per_block
+                               twice team_lanes / 32 the BDF runs twice as many lanes a cell) */
   int register_budget;      /* with warps_per_block > 0: 2 (<= 128 registers) or 1 (<= 255) */
   /* ReactorArkode (ReactorArkode.cpp:10-20, ReactorArkode.H:131-137) */
   int rk_method;            /* ode.rk_method, 40 (ZONNEVELD_5_3_4); box path only, as in the reference */

@@ -287,7 +287,10 @@ __device__ double reactor_rhs_srk(
   return T;
 }
 
-// Reactor Jacobian, column-major n x n: J[i*n + k] = d f_k / d y_i.
+// Reactor Jacobian, column-major n x n: J[i*n + k] = d f_k / d y_i.  Out of
+// line: inlined into the integrator the lanes of its column loops, which have
+// different lengths, ran one after another (100 drm19 cells, one warp a block:
+// 7.9 ms a call against 5.1).
 template <int TEAM, int PER>
 __device__ __noinline__ void reactor_jac(
   const Team<TEAM>& tm, const DevMech& M, int rtype, const double* y, double* J, double* sc, double* g,
@@ -1313,10 +1316,10 @@ struct Bdf {
   // time, input and output and the phase that takes its result; so the kernel
   // holds one copy of the right-hand side (and of the Newton iteration, the
   // factorisation and the solve), and warps that meet at the rendezvous run
-  // the same instructions whatever they need f for.  With a copy at each of
-  // the integrator's five call sites, the 16-warp drm19 kernel ran 520k cells/s
-  // (64^3 field) against 890k with them shared: its warps fetched different
-  // copies.
+  // the same instructions whatever they need f for.  With a copy inlined at
+  // each of the integrator's five call sites, the 16-warp drm19 kernel ran
+  // 520k cells/s (64^3 field), its warps fetching different copies; with one
+  // out of line, reading through generic pointers, 1.02M; as here 1.21M.
   enum : int { EV_START, EV_HIN, EV_NEWTON_FIRST, EV_NEWTON, EV_RESET, EV_JCOL };
 
   // fresh: integrate from w.zn (initial y, team-shared) towards tout --

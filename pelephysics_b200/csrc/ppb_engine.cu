@@ -382,7 +382,7 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
   set_off(dm.jg_off, off_joff);
   set_off(dm.jg_rx, off_jrx);
   set_off(dm.jg_c, off_jc);
-  // packed reaction records, fall-off records and efficiency masks
+  // packed reaction records and fall-off records
   const size_t off_rxp = (pk.used + 15) & ~size_t(15);
   int nfo = 0;
   for (int r = 0; r < R; r++)
@@ -393,8 +393,7 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
       nalpha++;
   const size_t off_fop = off_rxp + (size_t)R * sizeof(RxPack);
   const size_t off_fow = off_fop + (size_t)nfo * sizeof(FoPack);
-  const size_t off_msk = off_fow + (size_t)nfo * sizeof(FoPack);
-  const size_t off_effd = off_msk + (size_t)R * 4 * sizeof(unsigned);
+  const size_t off_effd = off_fow + (size_t)nfo * sizeof(FoPack);
   int fo = 0, aslot = 0;
   for (int r = 0; r < R; r++) {
     RxPack p;
@@ -503,9 +502,6 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
       p.aslot = (unsigned short)aslot++;
     }
     pk.put(off_rxp + r * sizeof(RxPack), &p, 1);
-    unsigned m[4] = {0, 0, 0, 0};
-    for (int e = t->eff_off[r]; e < t->eff_off[r + 1]; e++) m[t->eff_sp[e] >> 5] |= 1u << (t->eff_sp[e] & 31);
-    pk.put(off_msk + r * 4 * sizeof(unsigned), m, 4);
   }
   if (N > 127 || nfo > 254) pk.overflow = true;
   pk.used = off_effd + (size_t)nalpha * N * sizeof(double);
@@ -651,7 +647,6 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
   set_off(dm.fow, off_fow);
   set_off(dm.rxp, off_rxp);
   set_off(dm.fop, off_fop);
-  set_off(dm.effmask, off_msk);
   pack_rates(t, pk, dm);
   // SRK parameters (zeros for a mechanism without them)
   const double* srk = find_srk(t->name);

@@ -85,7 +85,6 @@ struct DevMech {
   // packed per-reaction records (see RxPack) for the warp-cooperative paths
   const struct RxPack* rxp;
   const struct FoPack* fop;
-  const unsigned* effmask; // 4 words per reaction: species with a listed efficiency
   const double* effd;      // [third-body reactions][nsp] efficiencies, 1 where unlisted
   // the Jacobian's columns: for species k, in reaction order, the reactions
   // whose d q_r / d c_k can be nonzero (every third-body / fall-off reaction
