@@ -78,17 +78,30 @@ def cpu_sample_index(ncells, n):
     return np.sort(np.random.default_rng(7).permutation(ncells)[:n])
 
 
+def ref_kernels(po, mech):
+    """1 where the reference's compiled kernels of the mechanism are built
+    (oracle/_ref; they need the reference's source), else 0: the oracle's own
+    table-driven kernels."""
+    return int(po.have_ref(mech))
+
+
+def oracle_kind(po, mech):
+    return "the reference's own compiled mechanism kernels (oracle/_ref)" if ref_kernels(po, mech) else \
+        "the oracle's table-driven kernels (the reference's are not built here)"
+
+
 def run_cpu(po, cells, idx, nthreads=0):
-    """The oracle (reference kernels) on cells[idx]; returns (seconds, rY,
-    flag, per-cell counters [steps, RHS, Jacobians, factorisations, Newton
-    iterations, error-test failures, convergence failures])."""
-    po.load_ref(MECH)
+    """The oracle (over the reference's kernels where they are built) on
+    cells[idx]; returns (seconds, rY, flag, per-cell counters [steps, RHS,
+    Jacobians, factorisations, Newton iterations, error-test failures,
+    convergence failures])."""
     rY = cells.rY[idx].copy()
     rX = cells.rX[idx].copy()
     src = np.ascontiguousarray(cells.rYsrc[idx])
     rXs = cells.rX_src[idx].copy()
     t0 = time.perf_counter()
-    flag, st, stats = po.react_flat_stats(MECH, 1, rY, src, rX, rXs, DT, use_ref_kernels=1, nthreads=nthreads, **OPTS)
+    flag, st, stats = po.react_flat_stats(MECH, 1, rY, src, rX, rXs, DT, use_ref_kernels=ref_kernels(po, MECH),
+                                          nthreads=nthreads, **OPTS)
     return time.perf_counter() - t0, rY, flag, stats
 
 
@@ -99,6 +112,11 @@ def reference_arm(args):
     from oracle import pyoracle as po
     from pelephysics_b200 import workloads as wl
 
+    if not po.have_ref(MECH):
+        print(json.dumps({"impl": "reference", "unavailable": f"the reference's {MECH} kernels are not built "
+                          f"({os.path.relpath(po.ref_path(MECH))}; oracle/build_ref.sh needs the reference's source)"}),
+              flush=True)
+        return 0
     eos, species, mw = oracle_eos(po, MECH)
     cells = wl.drm19_field(64, eos=eos, species=species, mw=mw)
     idx = cpu_sample_index(cells.ncells, CPU_SAMPLE)
@@ -367,23 +385,25 @@ def our_arm(args):
 
         idx = cpu_sample_index(n, CPU_SAMPLE)
         secs, y_cpu, flag, ostats = run_cpu(po, cells, idx)
-        cpu = {"value": len(idx) / secs, "unit": "cells/s", "cores": os.cpu_count(), "kind": "reference",
+        ref = ref_kernels(po, MECH)
+        cpu = {"value": len(idx) / secs, "unit": "cells/s", "cores": os.cpu_count(),
+               "kind": "reference" if ref else "oracle",
                "sample": f"{len(idx)} seeded cells of the same 64^3 field, one react; CVODE-algorithm BDF "
-                         "(oracle/reactor.c) over the reference's own compiled drm19 kernels (oracle/_ref), "
+                         f"(oracle/reactor.c) over {oracle_kind(po, MECH)}, "
                          "OpenMP over all host threads (ReactorCvode needs the absent SUNDIALS)"}
         # algorithmic work per cell from the oracle's counters on the sample
         # (implementation-independent), times the cells of the field
         flops = algorithmic_flops(ostats, N + 1) / len(idx) * n
         inputs = (cells.rY[idx], cells.rYsrc[idx], cells.rX[idx], cells.rX_src[idx])
-        acc = po.compare_to_reference(MECH, 1, *inputs, DT, y_gpu[idx], y_cpu, use_ref_kernels=1, **OPTS)
-        acc["fp32_factor"] = po.compare_to_reference(MECH, 1, *inputs, DT, y_fp32[idx], y_cpu, use_ref_kernels=1,
+        acc = po.compare_to_reference(MECH, 1, *inputs, DT, y_gpu[idx], y_cpu, use_ref_kernels=ref, **OPTS)
+        acc["fp32_factor"] = po.compare_to_reference(MECH, 1, *inputs, DT, y_fp32[idx], y_cpu, use_ref_kernels=ref,
                                                      **OPTS)
-        acc["plain"] = po.compare_to_reference(MECH, 1, *inputs, DT, y_plain[idx], y_cpu, use_ref_kernels=1, **OPTS)
+        acc["plain"] = po.compare_to_reference(MECH, 1, *inputs, DT, y_plain[idx], y_cpu, use_ref_kernels=ref, **OPTS)
         # against a converged solution (the oracle at rtol = atol = 1e-13):
         # the error of the GPU and of the oracle itself at 1e-10
         yconv = cells.rY[idx].copy()
         po.react_flat(MECH, 1, yconv, np.ascontiguousarray(cells.rYsrc[idx]), cells.rX[idx].copy(),
-                      cells.rX_src[idx].copy(), DT, use_ref_kernels=1, rtol=1e-13, atol=1e-13, max_order=5)
+                      cells.rX_src[idx].copy(), DT, use_ref_kernels=ref, rtol=1e-13, atol=1e-13, max_order=5)
         Yv = po.mass_fraction_rows(yconv, N)
         err = lambda yy: {"max_rel_T": float(np.max(np.abs(yy[:, N] - yconv[:, N]) / yconv[:, N])),
                           "max_abs_Y": float(np.abs(po.mass_fraction_rows(yy, N) - Yv).max())}
@@ -560,7 +580,7 @@ def measure_config(config, steps, sample):
     yc = cells.rY[idx].copy()
     t0 = time.perf_counter()
     flag, _, _ = po.react_flat(mech, 1, yc, np.ascontiguousarray(cells.rYsrc[idx]), cells.rX[idx].copy(),
-                               cells.rX_src[idx].copy(), cells.dt, use_ref_kernels=1, **opts)
+                               cells.rX_src[idx].copy(), cells.dt, use_ref_kernels=ref_kernels(po, mech), **opts)
     cpu_s = time.perf_counter() - t0
     out = {}
     for name, integ, extra in arms:
@@ -601,7 +621,7 @@ def measure_config(config, steps, sample):
             # the oracle's RK64 on the sample: the explicit scheme's own answer
             yk = cells.rY[idx].copy()
             po.react_flat(mech, 1, yk, np.ascontiguousarray(cells.rYsrc[idx]), cells.rX[idx].copy(),
-                          cells.rX_src[idx].copy(), cells.dt, method=1, use_ref_kernels=1, **opts)
+                          cells.rX_src[idx].copy(), cells.dt, method=1, use_ref_kernels=ref_kernels(po, mech), **opts)
             okk = np.all(np.isfinite(yk), axis=1)
             both = okk & ok
             out[name]["oracle_rk64_nonfinite_in_sample"] = int(np.sum(~okk))
@@ -611,7 +631,7 @@ def measure_config(config, steps, sample):
         r.close()
     return {"workload": workload, "cells": n, "opts": opts, "arms": out,
             "oracle_sample": {"cells": int(len(idx)), "seconds": cpu_s, "flag": int(flag),
-                              "kind": "oracle BDF over the reference's compiled kernels (oracle/_ref), OpenMP"}}
+                              "kind": f"oracle BDF over {oracle_kind(po, mech)}, OpenMP"}}
 
 
 def measure_lidryer(po, dev):
@@ -630,7 +650,7 @@ def measure_lidryer(po, dev):
     yc = cells.rY.copy()
     t0 = time.perf_counter()
     flag, _, _ = po.react_flat("LiDryer", 1, yc, np.ascontiguousarray(cells.rYsrc), cells.rX.copy(),
-                               cells.rX_src.copy(), cells.dt, use_ref_kernels=1, **opts)
+                               cells.rX_src.copy(), cells.dt, use_ref_kernels=ref_kernels(po, "LiDryer"), **opts)
     cpu_s = time.perf_counter() - t0
     out = {"workload": "LiDryer 16^3 (4096 cells), 1 atm, T 1000+400 U, phi 0.5+1.5 U, dt 1e-4 s, "
                        "rtol=atol=1e-10, BDF q<=5", "cells": n,
@@ -654,7 +674,7 @@ def measure_lidryer(po, dev):
         ms = a.elapsed_time(b)
         yg = y.cpu().numpy().T.copy()
         acc = po.compare_to_reference("LiDryer", 1, cells.rY, cells.rYsrc, cells.rX, cells.rX_src, cells.dt, yg, yc,
-                                      use_ref_kernels=1, **opts)
+                                      use_ref_kernels=ref_kernels(po, "LiDryer"), **opts)
         out[name] = {"cells_per_s": n / (ms / 1e3), "ms_per_react": ms, "accuracy_vs_fp64_oracle": acc}
         r.close()
     out["tuned_vs_plain"] = out["tuned"]["cells_per_s"] / out["plain"]["cells_per_s"]
@@ -681,7 +701,7 @@ def measure_qss(po, dev, sample=1024):
     yc = np.ascontiguousarray(cells.rY[idx])
     t0 = time.perf_counter()
     flag, _, _ = po.react_flat(mech, 1, yc, np.ascontiguousarray(cells.rYsrc[idx]), cells.rX[idx].copy(),
-                               cells.rX_src[idx].copy(), cells.dt, use_ref_kernels=1, **opts)
+                               cells.rX_src[idx].copy(), cells.dt, use_ref_kernels=ref_kernels(po, mech), **opts)
     cpu_s = time.perf_counter() - t0
     out = {"workload": f"{mech} {n} e-reactors, 1 atm, T 1100+1000 U, phi 0.5+0.5 U, dt 1e-5 s, rtol=atol=1e-10, "
                        "BDF q<=5, difference-quotient Jacobian", "cells": n,
@@ -705,7 +725,7 @@ def measure_qss(po, dev, sample=1024):
     ms = a.elapsed_time(b)
     yg = y.cpu().numpy().T.copy()[idx]
     acc = po.compare_to_reference(mech, 1, cells.rY[idx], cells.rYsrc[idx], cells.rX[idx], cells.rX_src[idx],
-                                  cells.dt, yg, yc, use_ref_kernels=1, **opts)
+                                  cells.dt, yg, yc, use_ref_kernels=ref_kernels(po, mech), **opts)
     wpb, team, regs, _ = r.launch_config()
     out["tuned"] = {"cells_per_s": n / (ms / 1e3), "ms_per_react": ms, "accuracy_vs_fp64_oracle": acc,
                     "launch": {"warps_per_block": wpb, "lanes_per_cell": team}}
