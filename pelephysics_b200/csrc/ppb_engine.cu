@@ -53,7 +53,8 @@ struct Packer {
   char* buf;     // destination image (nullptr: size only)
   size_t cap;    // capacity of buf
   size_t used = 0;
-  bool overflow = false;
+  bool overflow = false; // does not fit buf, or is beyond the limits of RxPack
+  int wide = 0;          // DevMech::wide
   template <typename T>
   size_t add(const T* p, size_t n)
   {
@@ -87,6 +88,43 @@ void set_off(const T*& field, size_t off)
 }
 } // namespace
 
+// A coefficient as a sum of doubles that are zero below their top 16 bits
+// (whole numbers up to 31 are one, a full significand is eleven): returns the
+// first, leaves the rest in c.
+static unsigned coefficient_part(double& c)
+{
+  unsigned long long bits;
+  memcpy(&bits, &c, 8);
+  bits &= 0xffffull << 48;
+  double top;
+  memcpy(&top, &bits, 8);
+  c -= top; // exact
+  return (unsigned)(bits >> 48);
+}
+
+static int coefficient_parts(double c)
+{
+  int n = 0;
+  do {
+    coefficient_part(c);
+    n++;
+  } while (c != 0.0 && n < 11);
+  return n;
+}
+
+// The entries (DevMech::wg, jh) of reaction r's coefficient c in species s's
+// list, from its k-th on; returns their number.
+static int put_coefficient(Packer& pk, size_t off, int N, int s, int k, int r, double c)
+{
+  int n = 0;
+  do {
+    const unsigned e = coefficient_part(c) << 16 | (unsigned)r;
+    pk.put(off + ((size_t)(k + n) * N + s) * sizeof(unsigned), &e, 1);
+    n++;
+  } while (c != 0.0 && n < 11);
+  return n;
+}
+
 // The rate records (RxRate) and the efficiency lists of the third-body and
 // fall-off reactions, in the layouts of DevMech.
 static void pack_rates(const PPBMechTables* t, Packer& pk, DevMech& dm)
@@ -104,35 +142,37 @@ static void pack_rates(const PPBMechTables* t, Packer& pk, DevMech& dm)
     neff = n > neff ? n : neff;
   }
   neff = (neff + EFF_UNROLL - 1) / EFF_UNROLL * EFF_UNROLL;
-  if (nal > 255 || R > 65535) pk.overflow = true;
+  if (R > 65535) pk.overflow = true;
   dm.nal = nal;
   dm.neff = neff;
   const size_t off_rr = (pk.used + 15) & ~size_t(15);
   const size_t off_m1 = off_rr + (size_t)R * sizeof(RxRate);
   const size_t off_sp = off_m1 + (size_t)neff * nal * sizeof(double);
+  bool wide; // the reaction does not fit RxRate
   // the slots of a phase space: a repeated species first (see RxRate)
   auto slots = [&](const int* sp, const double* c, int n, unsigned char (&out)[3]) {
     int k = 0, runs = 0, repeats = 0;
     for (int pass = 0; pass < 2; pass++)
       for (int j = 0; j < n; j++) {
         const int o = (int)c[j];
-        if ((double)o != c[j] || o < 1) pk.overflow = true;
+        if ((double)o != c[j] || o < 1) wide = true;
         if ((o > 1) != (pass == 0)) continue;
         runs++;
         repeats += (o > 1);
         for (int q = 0; q < o; q++)
           if (k < 3) out[k++] = (unsigned char)sp[j];
-          else pk.overflow = true;
+          else wide = true;
       }
     // a single repeated run is a factor of its own only next to one other
     // run, or in front of them in species order
-    if (repeats > 1 || (repeats == 1 && runs > 2 && (int)c[0] < 2)) pk.overflow = true;
+    if (repeats > 1 || (repeats == 1 && runs > 2 && (int)c[0] < 2)) wide = true;
     while (k < 3) out[k++] = (unsigned char)N;
   };
   int a = 0, fo = 0;
   for (int r = 0; r < R; r++) {
     RxRate p;
     memset(&p, 0, sizeof(p));
+    wide = false;
     p.A = t->rx_A[r];
     p.beta = t->rx_beta[r];
     p.EaR = t->rx_EaR[r];
@@ -141,19 +181,21 @@ static void pack_rates(const PPBMechTables* t, Packer& pk, DevMech& dm)
     for (int j = 0; j < 5; j++) p.kcs[j] = (unsigned char)N;
     if (t->rx_rev[r]) { // the reverse tables are read for a reversible reaction only
       slots(t->rx_rps_sp + r * PPB_MAXPS, t->rx_rps_c + r * PPB_MAXPS, t->rx_rps_n[r], p.rsp);
-      if (t->rx_kc_n[r] > 5) pk.overflow = true;
+      if (t->rx_kc_n[r] > 5) wide = true;
       for (int j = 0; j < t->rx_kc_n[r] && j < 5; j++) {
         unsigned long long bits;
         memcpy(&bits, &t->rx_kc_c[r * PPB_MAXKC + j], 8);
-        if (bits << 16) pk.overflow = true; // more than the top 16 bits of the double
+        if (bits << 16) wide = true; // more than the top 16 bits of the double
         p.kcs[j] = (unsigned char)t->rx_kc_sp[r * PPB_MAXKC + j];
         p.kch[j] = (unsigned short)(bits >> 48);
       }
-      if (t->rx_kcpow[r] < -1 || t->rx_kcpow[r] > 30) pk.overflow = true;
+      if (t->rx_kcpow[r] < -1 || t->rx_kcpow[r] >= RR_WIDE - 1) wide = true;
     }
+    if (third(r) && a > 255) wide = true;
+    if (wide) pk.wide |= WIDE_RATES;
     p.flags = (unsigned char)((t->rx_rev[r] ? RR_REV : 0) | (third(r) ? RR_ALPHA : 0) |
                               (t->nqss > 0 && t->rx_rmfwd[r] ? RR_RMF : 0) |
-                              ((t->rx_rev[r] ? t->rx_kcpow[r] + 1 : 1) << RR_KCPOW));
+                              ((wide ? RR_WIDE : t->rx_rev[r] ? t->rx_kcpow[r] + 1 : 1) << RR_KCPOW));
     p.fo = 255;
     if (t->rx_kind[r] == PPB_RX_TROE || t->rx_kind[r] == PPB_RX_LINDEMANN) p.fo = (unsigned char)fo++;
     if (third(r)) {
@@ -200,13 +242,12 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
   PPB_ADD(tmid, t->tmid, NT);
   // thermo polynomials, coefficient-major (th_row, th_at)
   const int ld = thermo_ld(N);
-  if (NT > ld) pk.overflow = true;
   auto add_thermo = [&](const double* src, int nc) {
     const size_t off = (pk.used + 15) & ~size_t(15);
     for (int k = 0; k < nc; k++)
       for (int g = 0; g < 2; g++)
         for (int s = 0; s < ld; s++) {
-          const double v = s < NT ? src[(2 * s + g) * nc + k] : 0.0;
+          const double v = s < N ? src[(2 * s + g) * nc + k] : 0.0;
           pk.put(off + ((size_t)(2 * k + g) * ld + s) * sizeof(double), &v, 1);
         }
     pk.used = off + (size_t)2 * nc * ld * sizeof(double);
@@ -218,6 +259,16 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
   set_off(dm.th_u, add_thermo(t->th_u, 6));
   set_off(dm.th_h, add_thermo(t->th_h, 6));
   set_off(dm.th_g, add_thermo(t->th_g, 7));
+  {
+    const int Q = t->nqss;
+    const size_t off = (pk.used + 15) & ~size_t(15);
+    for (int k = 0; k < 7; k++)
+      for (int g = 0; g < 2; g++)
+        for (int q = 0; q < Q; q++)
+          pk.put(off + ((size_t)(2 * k + g) * Q + q) * sizeof(double), &t->th_g[(2 * (N + 1 + q) + g) * 7 + k], 1);
+    pk.used = off + (size_t)14 * Q * sizeof(double);
+    set_off(dm.th_gq, off);
+  }
   {
     // e/(RT W) and h/(RT W) at the T solve's bounds
     const size_t off = (pk.used + 15) & ~size_t(15);
@@ -295,7 +346,8 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
   for (int s = 0; s < N; s++) {
     int cnt = 0;
     for (int r = 0; r < R; r++)
-      for (int j = 0; j < t->rx_wup_n[r]; j++) cnt += (t->rx_wup_sp[r * PPB_MAXW + j] == s);
+      for (int j = 0; j < t->rx_wup_n[r]; j++)
+        if (t->rx_wup_sp[r * PPB_MAXW + j] == s) cnt += coefficient_parts(t->rx_wup_c[r * PPB_MAXW + j]);
     longest = cnt > longest ? cnt : longest;
   }
   const int wgl = (longest + WG_UNROLL - 1) / WG_UNROLL * WG_UNROLL + WG_UNROLL;
@@ -307,12 +359,7 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
     for (int r = 0; r < R; r++) {
       for (int j = 0; j < t->rx_wup_n[r]; j++) {
         if (t->rx_wup_sp[r * PPB_MAXW + j] != s) continue;
-        unsigned long long bits;
-        memcpy(&bits, &t->rx_wup_c[r * PPB_MAXW + j], 8);
-        if (bits << 16) pk.overflow = true; // more than the top 16 bits of the double
-        const unsigned e = (unsigned)(bits >> 48) << 16 | (unsigned)r;
-        pk.put(off_g + ((size_t)k * N + s) * sizeof(unsigned), &e, 1);
-        k++;
+        k += put_coefficient(pk, off_g, N, s, k, r, t->rx_wup_c[r * PPB_MAXW + j]);
       }
     }
     pk.put(off_gn + s * sizeof(int), &k, 1);
@@ -351,7 +398,8 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
       int c = 0;
       for (int r = 0; r < R; r++)
         for (int j = 0; j < t->rx_jn_n[r]; j++)
-          c += (t->rx_jn_sp[r * PPB_MAXJN + j] == sp && t->rx_jn_c[r * PPB_MAXJN + j] != 0.0);
+          if (t->rx_jn_sp[r * PPB_MAXJN + j] == sp && t->rx_jn_c[r * PPB_MAXJN + j] != 0.0)
+            c += coefficient_parts(t->rx_jn_c[r * PPB_MAXJN + j]);
       jl = c > jl ? c : jl;
     }
     const size_t off_n = (pk.used + 15) & ~size_t(15);
@@ -362,12 +410,7 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
         for (int j = 0; j < t->rx_jn_n[r]; j++) {
           const double nu = t->rx_jn_c[r * PPB_MAXJN + j];
           if (t->rx_jn_sp[r * PPB_MAXJN + j] != sp || nu == 0.0) continue;
-          unsigned long long bits;
-          memcpy(&bits, &nu, 8);
-          if (bits << 16) pk.overflow = true;
-          const unsigned e = (unsigned)(bits >> 48) << 16 | (unsigned)r;
-          pk.put(off_e + ((size_t)c * N + sp) * sizeof(unsigned), &e, 1);
-          c++;
+          c += put_coefficient(pk, off_e, N, sp, c, r, nu);
         }
       pk.put(off_n + sp * sizeof(int), &c, 1);
       for (; c < jl; c++) {
@@ -539,9 +582,9 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
         }
         for (; o > 0; o--)
           if (q < 2) f[q++] = (unsigned char)sp[j];
-          else pk.overflow = true;
+          else pk.wide |= WIDE_JAC;
       }
-      if (mult > 15) pk.overflow = true;
+      if (mult > 15) pk.wide |= WIDE_JAC;
       return mult;
     };
     int e = 0;
@@ -579,7 +622,7 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
           unsigned long long bits;
           memcpy(&bits, &t->rx_jn_c[r * PPB_MAXJN + j], 8);
           if (m >= 5 || (bits << 16)) {
-            pk.overflow = true;
+            pk.wide |= WIDE_JAC;
             break;
           }
           je.nu[m] = (unsigned short)(bits >> 48);
@@ -648,6 +691,7 @@ static size_t pack_all(const PPBMechTables* t, Packer& pk, DevMech& dm)
   set_off(dm.rxp, off_rxp);
   set_off(dm.fop, off_fop);
   pack_rates(t, pk, dm);
+  dm.wide = pk.wide;
   // SRK parameters (zeros for a mechanism without them)
   const double* srk = find_srk(t->name);
   std::vector<double> nosrk;
@@ -675,7 +719,7 @@ int pack_mechanism(const PPBMechTables* t, char* buf, size_t cap, const void* de
   pack_all(t, pk, dm);
   if (pk.overflow) return -1;
   const char* b = (const char*)dev_base;
-  // every pointer member of DevMech follows the two ints
+  // every pointer member of DevMech follows the ints
   const size_t first = offsetof(DevMech, mw);
   const size_t count = (sizeof(DevMech) - first) / sizeof(void*);
   for (size_t i = 0; i < count; i++) {

@@ -410,7 +410,8 @@ static int occupancy_ns(const DevMech& M, int method, const LaunchConfig& lc)
 }
 
 template <int TEAM, int PER>
-__global__ void k_ajacobian(DevMech M, const double* sc, const double* T, int consP, double* J, int ncells)
+__global__ void k_ajacobian(const __grid_constant__ DevMech M, const double* sc, const double* T, int consP, double* J,
+                            int ncells)
 {
   extern __shared__ __align__(16) double psm[];
   Team<TEAM> tm;

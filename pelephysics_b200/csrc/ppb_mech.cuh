@@ -39,15 +39,19 @@ struct DevMech {
   int nsp, nrxn;
   int nqss, nrq; // QSS species and reactions with one (PPBMechTables)
   int nfo, nal, neff; // fall-off reactions, third-body and fall-off reactions, the longest list of efficiencies
-  int pad_;
+  int wide; // WIDE_RATES: a reaction does not fit RxRate; WIDE_JAC: a reaction does not fit JcEntry
   const double *mw, *imw, *tmid;
-  // NASA-7 polynomials, coefficient-major: coefficient k of range g (0 below
-  // tmid) of species s at [(2 k + g) * thermo_ld(nsp) + s], so that lanes
-  // owning consecutive species load consecutive doubles
+  // NASA-7 polynomials of the transported species, coefficient-major:
+  // coefficient k of range g (0 below tmid) of species s at
+  // [(2 k + g) * thermo_ld(nsp) + s], so that lanes owning consecutive species
+  // load consecutive doubles
   const double *th_cv, *th_cp, *th_dcp, *th_u, *th_h, *th_g;
   // e_k / (RT W_k) (then h_k) of species k at the bounds of the T solve:
   // [u at 90 K | u at 4000 K | h at 90 K | h at 4000 K], thermo_ld(nsp) each
   const double* th_lim;
+  // g/RT of the QSS species: coefficient k of range g of QSS species q at
+  // [(2 k + g) * nqss + q]
+  const double* th_gq;
   const int *rx_kind, *rx_rev, *rx_kcpow;
   const double *rx_A, *rx_beta, *rx_EaR, *rx_sum_nuk;
   const int *fps_n, *fps_sp;
@@ -70,7 +74,8 @@ struct DevMech {
   const int* fo_i;
   // gather of the productionRate updates: species s adds, in reaction order,
   // c qdot[r] for entries wg[j nsp + s], j < wg_n[s]: the top 16 bits of the
-  // double c, then the reaction r in 16 bits (padded to the longest list,
+  // double c (a coefficient that needs more is split over several entries),
+  // then the reaction r in 16 bits (padded to the longest list,
   // rounded up to WG_UNROLL, and WG_UNROLL entries more)
   const int* wg_n;
   const unsigned* wg;
@@ -140,25 +145,31 @@ static_assert(sizeof(RxPack) == 80, "RxPack is five 16-byte words");
 // What a rate evaluation needs of one reaction, in 48 bytes (three 16-byte
 // words, stored word-major so that a warp's loads are contiguous: the 80-byte
 // records above, read by consecutive lanes, took 20 cache lines per load).
-// Phase spaces are at most three slots (checked when the tables are packed),
-// a repeated species first, so that the left-to-right product of the slots is
-// the product of the species' powers in species order, bit for bit.
+// Phase spaces are at most three slots, a repeated species first, so that the
+// left-to-right product of the slots is the product of the species' powers in
+// species order, bit for bit.  A reaction that does not fit (more slots, more
+// than five Gibbs terms or a coefficient of more than 16 bits, a power of
+// 1/refC outside -1..29, a third-body slot above 255; found when the tables
+// are packed) is marked RR_WIDE and takes them from its RxPack record, whose
+// limits decide what is accepted.
 struct alignas(16) RxRate {
   double A, beta, EaR;
   unsigned char fsp[3], rsp[3];
   unsigned char kcs[5];
-  unsigned char flags;   // RR_REV, RR_ALPHA, RR_RMF, and kcpow + 1 from bit RR_KCPOW
+  unsigned char flags;   // RR_REV, RR_ALPHA, RR_RMF, and kcpow + 1 (or RR_WIDE) from bit RR_KCPOW
   unsigned short kch[5]; // top 16 bits of the double coefficient of kcs
   unsigned char fo;      // fall-off record, 255 = none
   unsigned char al;      // third-body slot (al_m1, al_sp)
 };
 static_assert(sizeof(RxRate) == 48, "RxRate is three 16-byte words");
-enum { RR_REV = 1, RR_ALPHA = 2, RR_RMF = 4, RR_KCPOW = 3 };
+enum { RR_REV = 1, RR_ALPHA = 2, RR_RMF = 4, RR_KCPOW = 3, RR_WIDE = 31 };
+enum { WIDE_RATES = 1, WIDE_JAC = 2 }; // DevMech::wide
 
 // One reaction in one column of the Jacobian, in 32 bytes: the derivative of a
 // phase space is c * sc[s0] * sc[s1] (the factors in species order, the unit
 // slot where there are fewer), the net stoichiometry five species with the top
-// 16 bits of their coefficients as doubles (0: none).
+// 16 bits of their coefficients as doubles (0: none).  In a mechanism with a
+// reaction beyond that (WIDE_JAC) only r, flags and e are used.
 struct alignas(16) JcEntry {
   unsigned short r;
   unsigned char flags;     // JC_INR, JC_INP, JC_ALPHA, JC_LISTED
@@ -174,9 +185,8 @@ enum { JC_INR = 1, JC_INP = 2, JC_ALPHA = 4, JC_LISTED = 8 };
 constexpr int WG_UNROLL = 8;  // gather entries loaded together
 constexpr int EFF_UNROLL = 4; // efficiencies loaded together
 
-// Leading dimension of the thermo tables: the species, then (QSS mechanisms)
-// the unit slot and at most ten QSS species, rounded up to 32 bytes.
-__host__ __device__ constexpr int thermo_ld(int nsp) { return (nsp + 11 + 3) & ~3; }
+// Leading dimension of the thermo tables: the species, rounded up to 32 bytes.
+__host__ __device__ constexpr int thermo_ld(int nsp) { return (nsp + 3) & ~3; }
 
 struct alignas(16) FoPack {
   double P0, k0, beta0, EaR0, prdim, a, T3, T1, T2, oma, iT3, iT1;
@@ -439,6 +449,16 @@ __device__ __forceinline__ double g_RT(const DevMech& M, int s, double T, double
   const double T2 = T * T, T3 = T * T * T, T4 = T * T * T * T;
   return th_at<NS>(M, c, 0) * invT + th_at<NS>(M, c, 1) + th_at<NS>(M, c, 2) * logT + th_at<NS>(M, c, 3) * T +
          th_at<NS>(M, c, 4) * T2 + th_at<NS>(M, c, 5) * T3 + th_at<NS>(M, c, 6) * T4;
+}
+
+// g/RT of QSS species q (concentration slot nsp + 1 + q), the same formula
+__device__ __forceinline__ double g_RT_qss(const DevMech& M, int q, double T, double invT, double logT)
+{
+  const int ld = 2 * M.nqss;
+  const double* c = M.th_gq + (nasa_range(M, M.nsp + 1 + q, T) ? M.nqss : 0) + q;
+  const double T2 = T * T, T3 = T * T * T, T4 = T * T * T * T;
+  return __ldg(c) * invT + __ldg(c + ld) + __ldg(c + 2 * ld) * logT + __ldg(c + 3 * ld) * T + __ldg(c + 4 * ld) * T2 +
+         __ldg(c + 5 * ld) * T3 + __ldg(c + 6 * ld) * T4;
 }
 
 // Mixture energy (EH=0: CKUBMS, erg/g) or enthalpy (EH=1: CKHBMS) and the
@@ -806,56 +826,120 @@ __device__ __forceinline__ FoPack load_fow(const DevMech& M, int f)
   return p;
 }
 
-// Rates of progress q_f, q_r from a rate record (same formulas as rxn_qdot).
-__device__ __forceinline__ void rr_rates(const DevMech& M, const RxRate& p, double T, double invT, double logT,
+// The factor of a fall-off reaction's rate (third-body concentration Corr).
+__device__ __forceinline__ double falloff_corr(const FoPack& f, double Corr, double k_f, double T, double invT,
+                                               double logT)
+{
+  const double redP = Corr / k_f * f.P0 * ppb_exp(f.beta0 * logT - f.EaR0 * invT);
+  const double F = redP / (1.0 + redP);
+  if (f.lindemann) return F;
+  const double logPred = ppb_log10(redP);
+  double fc = 0.0;
+  if (f.p1) fc = f.oma * ppb_exp(-T * f.iT3);
+  if (f.p2) fc += f.a * ppb_exp(-T * f.iT1);
+  if (f.ntroe == 4) fc += ppb_exp(-f.T2 * invT);
+  const double logFcent = ppb_log10(fc);
+  const double troe_c = -0.4 - 0.67 * logFcent;
+  const double troe_n = 0.75 - 1.27 * logFcent;
+  const double troe = (troe_c + logPred) / (troe_n - 0.14 * (troe_c + logPred));
+  const double F_troe = ppb_exp(M_LN10 * logFcent / (1.0 + troe * troe));
+  return F * F_troe;
+}
+
+// Rates of progress q_f, q_r of reaction r from its rate record (same formulas
+// as rxn_qdot).  WIDE: the mechanism has RR_WIDE reactions; they read the
+// packed record in memory.  The caller's loop is there once with and once
+// without them: one loop that asks at each reaction took 1 to 2.5 % longer in
+// mechanisms that have none (lidryer box, ReactorArkode), and out of line it
+// cost the QSS kernel 500 bytes of spills and 9 %.
+template <bool WIDE>
+__device__ __forceinline__ void rr_rates(const DevMech& M, const RxRate& p, int r, double T, double invT, double logT,
                                          double refC, double refCinv, double mixture, const double* sc,
                                          const double* g, double& qf_out, double& qr_out)
 {
+  const bool wide = WIDE && (p.flags >> RR_KCPOW) == RR_WIDE;
+  const RxPack* w = M.rxp + r;
   const double k_f = p.A * ppb_exp(p.beta * logT - p.EaR * invT);
   double Corr = 1.0;
   const bool corr = (p.flags & RR_ALPHA) != 0;
   if (corr) {
     Corr = mixture;
+    const int al = wide ? (int)w->aslot : (int)p.al;
     for (int j = 0; j < M.neff; j += EFF_UNROLL) {
 #pragma unroll
       for (int q = 0; q < EFF_UNROLL; q++) {
-        const int e = (j + q) * M.nal + p.al;
+        const int e = (j + q) * M.nal + al;
         Corr += __ldg(M.al_m1 + e) * sc[__ldg(M.al_sp + e)];
       }
     }
   }
   if (p.fo != 255) {
-    const FoPack f = load_fow(M, p.fo);
-    const double redP = Corr / k_f * f.P0 * ppb_exp(f.beta0 * logT - f.EaR0 * invT);
-    const double F = redP / (1.0 + redP);
-    if (!f.lindemann) {
-      const double logPred = ppb_log10(redP);
-      double fc = 0.0;
-      if (f.p1) fc = f.oma * ppb_exp(-T * f.iT3);
-      if (f.p2) fc += f.a * ppb_exp(-T * f.iT1);
-      if (f.ntroe == 4) fc += ppb_exp(-f.T2 * invT);
-      const double logFcent = ppb_log10(fc);
-      const double troe_c = -0.4 - 0.67 * logFcent;
-      const double troe_n = 0.75 - 1.27 * logFcent;
-      const double troe = (troe_c + logPred) / (troe_n - 0.14 * (troe_c + logPred));
-      const double F_troe = ppb_exp(M_LN10 * logFcent / (1.0 + troe * troe));
-      Corr = F * F_troe;
-    } else {
-      Corr = F;
-    }
+    Corr = falloff_corr(load_fow(M, p.fo), Corr, k_f, T, invT, logT);
   }
-  const double phf = (sc[p.fsp[0]] * sc[p.fsp[1]]) * sc[p.fsp[2]];
+  double phf = (sc[p.fsp[0]] * sc[p.fsp[1]]) * sc[p.fsp[2]];
+  if (wide) {
+    phf = 1.0;
+#pragma unroll 1
+    for (int j = 0; j < 4; j++) phf *= sc[w->fsp[j]];
+  }
   const double qf = corr ? Corr * k_f * phf : k_f * phf;
   double qr = 0.0;
   if (p.flags & RR_REV) {
     double arg = 0.0;
 #pragma unroll
     for (int j = 0; j < 5; j++) arg += __hiloint2double((int)((unsigned)p.kch[j] << 16), 0) * g[p.kcs[j]];
-    const double phr = (sc[p.rsp[0]] * sc[p.rsp[1]]) * sc[p.rsp[2]];
-    qr = (corr ? Corr * k_f : k_f) * ppb_exp(-arg) * refc_pow((p.flags >> RR_KCPOW) - 1, refC, refCinv) * phr;
+    double phr = (sc[p.rsp[0]] * sc[p.rsp[1]]) * sc[p.rsp[2]];
+    int kcpow = (p.flags >> RR_KCPOW) - 1;
+    if (wide) {
+      arg = 0.0;
+#pragma unroll 1
+      for (int j = 0; j < 6; j++) arg += (double)w->kcc[j] * g[w->kcs[j]];
+      phr = 1.0;
+#pragma unroll 1
+      for (int j = 0; j < 8; j++) phr *= sc[w->rsp[j]];
+      kcpow = w->kcpow;
+    }
+    qr = (corr ? Corr * k_f : k_f) * ppb_exp(-arg) * refc_pow(kcpow, refC, refCinv) * phr;
   }
   qf_out = (p.flags & RR_RMF) ? 0.0 : qf;
   qr_out = qr;
+}
+
+// The species columns of the Jacobian (ajacobian_packed, pass 3) of a mechanism
+// with a reaction that does not fit JcEntry, from the RxPack records.
+template <int TEAM>
+__device__ __noinline__ void jac_columns_wide(Team<TEAM> tm, const DevMech& M, double* J, const double* sc, int consP,
+                                              const double* jx)
+{
+  const int N = M.nsp, n = N + 1;
+  for (int k = tm.lane; k < N; k += TEAM) {
+    double dq = 0.0;
+    double* Jk = J + k * n;
+    const int cnt = __ldg(M.jc_n + k);
+    for (int j = 0; j < cnt; j++) {
+      JcEntry e;
+      reinterpret_cast<int4*>(&e)[0] = __ldg(M.jc + (2 * j) * N + k);
+      const RxPack p = load_rx(M, e.r);
+      const double k_f = jx[4 * e.r + 0], k_r = jx[4 * e.r + 1], fac = jx[4 * e.r + 2];
+      const bool inr = slots_has(p.fsp, k), inp = p.rev && slots_has(p.rsp, k);
+      const bool alpha = (e.flags & JC_ALPHA) != 0;
+      double d = 0.0;
+      if (alpha) {
+        const double ef = consP == 1 ? e.e - 1 : e.e;
+        if (consP == 1 ? (e.flags & JC_LISTED) != 0 : ef != 0.0) d = ef * fac;
+      }
+      if (inr) d += k_f * slots_dproduct(p.fsp, sc, k);
+      if (inp) d -= k_r * slots_dproduct(p.rsp, sc, k);
+      if (alpha && consP != 1) {
+        if (e.e == 0.0 && !inr && !inp) d = dq;
+        dq = d;
+      }
+#pragma unroll
+      for (int q = 0; q < 6; q++)
+        if (q < p.njn && p.jnc[q]) Jk[p.jns[q]] += (double)p.jnc[q] * d;
+    }
+  }
+  tm.sync();
 }
 
 // Scratch doubles of the QSS solve: the coefficients q_f,k, q_r,k (2 nrq)
@@ -883,14 +967,15 @@ __device__ void qss_solve(const Team<TEAM>& tm, const DevMech& M, double* sc, do
   const int N = M.nsp, Q = M.nqss, K = M.nrq, W = Q + 1;
   constexpr double eps = 1e-12;
   for (int q = tm.lane; q < Q; q += TEAM) {
-    g[N + 1 + q] = g_RT(M, N + 1 + q, T, invT, logT);
+    g[N + 1 + q] = g_RT_qss(M, q, T, invT, logT);
     sc[N + 1 + q] = 1.0;
   }
   tm.sync();
   for (int k = tm.lane; k < K; k += TEAM) {
-    const RxRate p = load_rr(M, __ldg(M.q_rx + k));
+    const int r = __ldg(M.q_rx + k);
+    const RxRate p = load_rr(M, r);
     double qf, qr;
-    rr_rates(M, p, T, invT, logT, refC, refCinv, mixture, sc, g, qf, qr);
+    rr_rates<true>(M, p, r, T, invT, logT, refC, refCinv, mixture, sc, g, qf, qr);
     co[2 * k] = qf;
     co[2 * k + 1] = qr;
   }
@@ -989,11 +1074,20 @@ __device__ __forceinline__ void production_rate_core(const Team<TEAM>& tm, const
                                                      double refC, double refCinv, double mixture, RateScratch& rs)
 {
   const int N = NS > 0 ? NS : M.nsp;
-  for (int r = tm.lane; r < M.nrxn; r += TEAM) {
-    const RxRate p = load_rr(M, r);
-    double qf, qr;
-    rr_rates(M, p, T, invT, logT, refC, refCinv, mixture, sc_in, rs.g, qf, qr);
-    rs.qd[r] = __dsub_rn(qf, qr); // both rounded: no contraction with either product
+  if (!(M.wide & WIDE_RATES)) {
+    for (int r = tm.lane; r < M.nrxn; r += TEAM) {
+      const RxRate p = load_rr(M, r);
+      double qf, qr;
+      rr_rates<false>(M, p, r, T, invT, logT, refC, refCinv, mixture, sc_in, rs.g, qf, qr);
+      rs.qd[r] = __dsub_rn(qf, qr); // both rounded: no contraction with either product
+    }
+  } else {
+    for (int r = tm.lane; r < M.nrxn; r += TEAM) {
+      const RxRate p = load_rr(M, r);
+      double qf, qr;
+      rr_rates<true>(M, p, r, T, invT, logT, refC, refCinv, mixture, sc_in, rs.g, qf, qr);
+      rs.qd[r] = __dsub_rn(qf, qr);
+    }
   }
   tm.sync();
   for (int s = tm.lane; s < N; s += TEAM) wdot[s] = rate_gather(M, N, s, rs.qd);
@@ -1327,10 +1421,11 @@ __device__ void ajacobian_packed(
   // walk needs of a reaction, one coalesced load ahead; from the reactions'
   // 80-byte records, with their slot lists searched for k, a column of drm19
   // took 2,000 instructions more than its arithmetic.
+  if (M.wide & WIDE_JAC) jac_columns_wide<TEAM>(tm, M, J, sc, consP, jx);
 #pragma unroll
   for (int qq = 0; qq < PER; qq++) {
     const int k = tm.lane + qq * TEAM;
-    if (k >= N) break;
+    if (k >= N || (M.wide & WIDE_JAC)) break;
     double dq = 0.0;
     double* Jk = J + k * n;
     const int cnt = __ldg(M.jc_n + k);
