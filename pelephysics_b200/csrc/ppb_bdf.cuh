@@ -1048,6 +1048,7 @@ struct Bdf {
     if constexpr (TEAM > 1) {
       ier = lu_factor_team<TEAM, LT, (n + Team<TEAM>::W - 1) / Team<TEAM>::W>(tm, w.A, n, w.piv) ? 1 : 0;
       if (!ier) {
+        // (FP32: w.perm is that column's place, entry by entry)
         for (int i = tm.lane; i < n; i += TEAM) w.perm[i] = (int)w.A[n * n + i];
         diag_recip(tm, w.A, w.dinv, n);
       }

@@ -59,6 +59,15 @@ def test_block_sizes_change_no_bits(cuda, oracle, mech, dt, ncells):
         assert np.array_equal(y, ref) and np.array_equal(s, st), form
 
 
+# five cells of 46,464 bytes in a block's 232,448
+def test_the_largest_fp32_block_fits(cuda, oracle):
+    cells = premix_oracle(oracle, "grimech30", 11, 3, 1300.0, 500.0, 0.5, 1.0)
+    opts = dict(rtol=1e-8, atol=1e-12, max_order=5, lu_fp32=1)
+    a, sa = _react("grimech30", *cells, 1e-6, warps_per_block=4, **opts)
+    b, sb = _react("grimech30", *cells, 1e-6, warps_per_block=5, **opts)
+    assert np.array_equal(a, b) and np.array_equal(sa, sb)
+
+
 # tiles of 32 cells (16 for 88 species)
 @pytest.mark.parametrize("n", [1, 15, 17, 33])
 @pytest.mark.parametrize("mech", ["LiDryer", "drm19", "dodecane_lu", "heptane_lu_88sk"])
