@@ -395,8 +395,10 @@ __device__ void jc_mul(const Team<TEAM>& tm, int n, const double* Jc, const doub
 }
 
 // FP64 LU of I - gamma Jc (transpose = false) or of its transpose (out of
-// line, as the solve below: the sweeps keep one copy of each).
-template <int TEAM, int PER>
+// line, as the solve below: the sweeps keep one copy of each).  NS species:
+// n = NS + 1 rows, which is a row a lane more than the species take when they
+// fill the lanes.
+template <int TEAM, int NS>
 __device__ __noinline__ int adj_factor(const Team<TEAM>& tm, int n, const double* Jc, double gamma, bool transpose,
                                        double* A, int* piv)
 {
@@ -409,7 +411,7 @@ __device__ __noinline__ int adj_factor(const Team<TEAM>& tm, int n, const double
     }
   }
   tm.sync();
-  return lu_factor_team<TEAM, double, PER>(tm, A, n, piv);
+  return lu_factor_team<TEAM, double, (NS + Team<TEAM>::W) / Team<TEAM>::W>(tm, A, n, piv);
 }
 
 template <int TEAM>
@@ -548,7 +550,7 @@ __device__ bool rev_linear(const Team<TEAM>& tm, int n, int qmax, const TapeRec&
 // tangent (forward) of the Nordsieck history, pend that of the last
 // correction.  lamE is the adjoint of E (reverse) and dE the tangent of E
 // (forward).
-template <int TEAM, int PER, typename LT>
+template <int TEAM, int NS, typename LT>
 struct AdjSweep {
   // the team and the workspaces by value: the sweeps are out of line, and their
   // object must not hold the address of the recording loop's workspace
@@ -564,7 +566,7 @@ struct AdjSweep {
   {
     for (int i = tm.lane; i < n; i += TEAM) a.ybuf[i] = yg[i];
     tm.sync();
-    return rhs_exact_jacobian<TEAM, PER, LT>(tm, M, o.reactor_type, t, a.ybuf, cin.rhoe, cin.rhoesrc, w.src, w, a);
+    return rhs_exact_jacobian<TEAM, (NS + TEAM - 1) / TEAM, LT>(tm, M, o.reactor_type, t, a.ybuf, cin.rhoe, cin.rhoesrc, w.src, w, a);
   }
 
   // ---- forward (tangent-linear)
@@ -607,7 +609,7 @@ struct AdjSweep {
         tangent_rhs(pt, a.lam, dE, dp, a.mu);
         for (int i = tm.lane; i < n; i += TEAM) a.mu[i] = gamma * a.mu[i] - rl1 * a.lam[n + i];
         tm.sync();
-        if (adj_factor<TEAM, PER>(tm, n, a.Jc, gamma, false, a.AT, a.piv)) return ST_ADJ_SINGULAR;
+        if (adj_factor<TEAM, NS>(tm, n, a.Jc, gamma, false, a.AT, a.piv)) return ST_ADJ_SINGULAR;
         adj_solve<TEAM>(tm, a.AT, n, a.piv, a.mu);
         for (int i = tm.lane; i < n; i += TEAM) {
           const double d = a.mu[i];
@@ -698,7 +700,7 @@ __host__ __device__ inline size_t item_bytes(int N, int R)
   return ((8 * (14 * n + 6 * (size_t)R + 2 * n * n) + 4 * n) + 15) & ~size_t(15);
 }
 
-template <int TEAM, int PER>
+template <int TEAM, int NS>
 __device__ void eval_item(const Team<TEAM>& tm, const DevMech& M, int rtype, double t, double gamma, const double* yg,
                           double rhoe, double rhoesrc, const double* srcg, char* smem, double* item,
                           const ItemLayout& IL)
@@ -729,9 +731,9 @@ __device__ void eval_item(const Team<TEAM>& tm, const DevMech& M, int rtype, dou
     w.src[i] = (i < N && srcg) ? srcg[i] : 0.0;
   }
   tm.sync();
-  const AdjPoint pt = rhs_exact_jacobian<TEAM, PER, double>(tm, M, rtype, t, a.ybuf, rhoe, rhoesrc, w.src, w, a);
+  const AdjPoint pt = rhs_exact_jacobian<TEAM, (NS + TEAM - 1) / TEAM, double>(tm, M, rtype, t, a.ybuf, rhoe, rhoesrc, w.src, w, a);
   int sing = 0;
-  if (gamma != 0.0) sing = adj_factor<TEAM, PER>(tm, n, a.Jc, gamma, true, a.AT, a.piv);
+  if (gamma != 0.0) sing = adj_factor<TEAM, NS>(tm, n, a.Jc, gamma, true, a.AT, a.piv);
   for (int i = tm.lane; i < n * n; i += TEAM) item[i] = a.Jc[i];
   if (gamma != 0.0)
     for (int i = tm.lane; i < n * n; i += TEAM) item[IL.at + i] = a.AT[i];

@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(512, 1) k_adj_seg(const __grid_constant__ DevM
     rec.close_rec = C.close_rec;
     rec.close_y = C.close_y;
     rec.begin();
-    AdjSweep<32, (NS + 31) / 32, LT> sw{tm, M, o, w, a, cin, n, o.max_order};
+    AdjSweep<32, NS, LT> sw{tm, M, o, w, a, cin, n, o.max_order};
     const double dE = (tangent && b.dE) ? b.dE[c] : 0.0;
     int nstloc = 0, ncp = 0, flag = ST_OK;
     bool done = false;
@@ -543,7 +543,6 @@ __global__ void __launch_bounds__(256) k_adj_items(DevMech M, int rtype, AdjBatc
   extern __shared__ __align__(16) char smem[];
   Team<32> tm;
   constexpr int n = NS + 1;
-  constexpr int PER = (NS + 31) / 32;
   const int warp = threadIdx.x / 32;
   const int i = i0 + blockIdx.x * (blockDim.x / 32) + warp;
   if (i >= i1) return;
@@ -569,7 +568,7 @@ __global__ void __launch_bounds__(256) k_adj_items(DevMech M, int rtype, AdjBatc
     gamma = sg.yinfo[2 * slot + 1];
   }
   const ItemLayout IL(NS, M.nrxn);
-  eval_item<32, PER>(tm, M, rtype, t, gamma, yg, b.rhoe[c], b.rhoesrc ? b.rhoesrc[c] : 0.0,
+  eval_item<32, NS>(tm, M, rtype, t, gamma, yg, b.rhoe[c], b.rhoesrc ? b.rhoesrc[c] : 0.0,
                      b.src ? b.src + (size_t)c * NS : nullptr, smem + (size_t)warp * warp_smem,
                      C.items + (size_t)(i - i0) * IL.stride, IL);
 }

@@ -401,6 +401,7 @@ __device__ __forceinline__ int lu_factor_team(const Team<TEAM>& tm, LT* A, int n
   constexpr int W = Team<TEAM>::W, NW = Team<TEAM>::NW;
   const int wl = tm.lane % W, wid = tm.lane / W;
   const unsigned mask = tm.mask;
+  if (n > W * RPL) return n + 1; // more rows than the lanes hold
   for (int i = tm.lane; i < n; i += TEAM) A[n * n + i] = (LT)i;
   LT held[RPL]; // the scaled column the warp still has to write (NW > 1)
 #pragma unroll
