@@ -61,13 +61,17 @@ typedef struct ppb_options {
   int warps_per_block;      /* tuned engine block size in warps (1, 2, 4, 8; 12 or 16 for the BDF, either LU
                                precision, with 32 lanes per cell and budget 2: one block per SM); 0 = autotune the block
                                size, lanes per cell and register budget on the first call (the SRK EOS and QSS
-                               mechanisms, not autotuned: 16 warps where 16 cells fit one SM, else <= 8) */
+                               mechanisms, not autotuned: 16 warps where 16 cells fit one SM, else <= 8).  The pick
+                               goes by time, and blocks of 16 warps and 16-lane teams round differently from the
+                               others (through ignition at rtol = 1e-10 that grows to 1e-8 of the result): fix the
+                               launch for the same bits from run to run */
   int use_graph;            /* replay react() as a captured CUDA graph, 1 */
   int adjoint_checkpoint_interval; /* accepted BDF steps between adjoint checkpoints, 16 */
   int adjoint_memory_mb;    /* device memory for adjoint checkpoints, tapes and points, 16384 */
   int team_lanes;           /* with warps_per_block > 0: lanes per cell, 32, 16 (<= 21 species), 64
-                               (33..64 species) or 128 (65..128 species; one cell per block; with warps_per_block
-                               twice team_lanes / 32 the BDF runs twice as many lanes a cell) */
+                               (33..64 species) or 128 (65..128 species); 64 and 128: one cell per block, of
+                               team_lanes / 32 warps whatever warps_per_block says.  The BDF with two lanes a
+                               species: 128 with warps_per_block 4 (33..64 species), 256 with 8 (65..128) */
   int register_budget;      /* with warps_per_block > 0: 2 (<= 128 registers) or 1 (<= 255) */
   /* ReactorArkode (ReactorArkode.cpp:10-20, ReactorArkode.H:131-137) */
   int rk_method;            /* ode.rk_method, 40 (ZONNEVELD_5_3_4); box path only, as in the reference */

@@ -1386,7 +1386,7 @@ int ppb_get_launch_config(ppb_reactor* r, int* warps_per_block, int* team_lanes,
   LaunchConfig tl;
   if (r->opt.warps_per_block <= 0) tuned_config(r, &tl, &ms);
   if (warps_per_block) *warps_per_block = lc.warps_per_block;
-  if (team_lanes) *team_lanes = (lc.team > 32 && lc.team == 2 * species_team(r->t->nsp)) ? lc.team / 2 : lc.team;
+  if (team_lanes) *team_lanes = lc.team;
   if (register_budget) *register_budget = lc.minb;
   if (tuned_ms) *tuned_ms = ms;
   return 0;

@@ -60,15 +60,17 @@ struct LaunchConfig {
 };
 // Lanes of the multi-warp team with one lane per species (0: none).
 inline int species_team(int nsp) { return nsp <= 21 ? 0 : nsp <= 64 ? 64 : 128; }
-// Lanes of a fixed launch (options warps_per_block = w, team_lanes = lanes):
-// lanes, or twice as many when w asks for twice lanes / 32 warps.  A team the
+// Lanes of a fixed launch (options warps_per_block = w, team_lanes = lanes).
+// The BDF's team of two lanes a species goes by its own lanes and warps (128
+// and 4, or 256 and 8), as ppb_get_launch_config reports it.  A team the
 // mechanism has not is refused at the launch (1024 lanes: no such kernel).
 inline int fixed_team(int nsp, int method, int w, int lanes)
 {
+  const int st = species_team(nsp);
   if (lanes == 16) return 16;
+  if (st > 0 && lanes == 2 * st && w == lanes / 32 && method == METHOD_BDF) return lanes;
   if (lanes != 64 && lanes != 128) return 32;
-  if (lanes != species_team(nsp)) return 1024;
-  return (method == METHOD_BDF && w == lanes / 16) ? 2 * lanes : lanes;
+  return lanes == st ? lanes : 1024;
 }
 // Resident cells per SM of the tuned kernel in configuration lc (0: the
 // configuration does not fit or is not compiled).

@@ -161,7 +161,9 @@ extern "C" int ppb_react_flat_device_noalloc(const char* mechanism, const char* 
                          "parameters");
   if (o.warps_per_block < 0 || o.warps_per_block > 16)
     return nf(PPB_E_ARG, "warps_per_block must be in 0..16 (0: the largest block of <= 8 warps that fits)");
-  if (o.team_lanes != 0 && o.team_lanes != 16 && o.team_lanes != 32 && o.team_lanes != 64 && o.team_lanes != 128)
+  const bool two_a_species = o.team_lanes == 256 && o.warps_per_block == 8 && species_team(t->nsp) == 128;
+  if (o.team_lanes != 0 && o.team_lanes != 16 && o.team_lanes != 32 && o.team_lanes != 64 && o.team_lanes != 128 &&
+      !two_a_species)
     return nf(PPB_E_ARG, "team_lanes must be 0, 16, 32, 64 or 128");
   if (o.register_budget != 0 && o.register_budget != 1 && o.register_budget != 2)
     return nf(PPB_E_ARG, "register_budget must be 0, 1 or 2");

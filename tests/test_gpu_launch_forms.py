@@ -59,6 +59,31 @@ def test_block_sizes_change_no_bits(cuda, oracle, mech, dt, ncells):
         assert np.array_equal(y, ref) and np.array_equal(s, st), form
 
 
+def _config(mech, **opts):
+    r = Reactor(mech)
+    r.init(1, 1, **opts)
+    cfg = r.launch_config()[:3]
+    r.close()
+    return cfg
+
+
+@pytest.mark.parametrize("mech,lanes,T0,P,dt", [("dodecane_lu", 64, 1000.0, 40 * 1013250.0, 2e-6),
+                                                ("heptane_lu_88sk", 128, 900.0, 20 * 1013250.0, 1e-5)])
+def test_a_fixed_team_keeps_its_lanes(cuda, oracle, mech, lanes, T0, P, dt):
+    """team_lanes is the lanes of a cell whatever warps_per_block says; two
+    lanes a species are asked for, and reported, as what they are."""
+    for wpb in (1, 2, 4, 8):
+        assert _config(mech, warps_per_block=wpb, team_lanes=lanes) == (lanes // 32, lanes, 1)
+    two = dict(warps_per_block=lanes // 16, team_lanes=2 * lanes)
+    assert _config(mech, **two) == (lanes // 16, 2 * lanes, 1)
+    cells = premix_oracle(oracle, mech, 5, 7, T0, 500.0, 0.5, 1.0, P=P)
+    opts = dict(rtol=1e-8, atol=1e-12, max_order=5)
+    for fp32 in (0, 1):
+        a, sa = _react(mech, *cells, dt, warps_per_block=1, team_lanes=lanes, lu_fp32=fp32, **opts)
+        b, sb = _react(mech, *cells, dt, lu_fp32=fp32, **two, **opts)
+        assert np.array_equal(a, b) and np.array_equal(sa, sb)
+
+
 # five cells of 46,464 bytes in a block's 232,448
 def test_the_largest_fp32_block_fits(cuda, oracle):
     cells = premix_oracle(oracle, "grimech30", 11, 3, 1300.0, 500.0, 0.5, 1.0)
