@@ -1,7 +1,9 @@
-"""Every launch form of the BDF kernels integrates a cell with the same
-arithmetic: teams of one and of two lanes a species, blocks of different sizes
-and batches that leave lanes, warps and blocks idle give the same bits.  And
-the transport kernel at the edges of its tiles."""
+"""Launch forms of the BDF kernels.  Teams of one and of two lanes a species,
+blocks of up to 12 warps and batches that leave lanes, warps and blocks idle
+give the same bits.  Blocks of 16 warps round the energy of one temperature
+solve an iteration differently, and 16-lane teams sum in another order where
+there are more unknowns than lanes: these agree to what rounding grows to.
+And the transport kernel at the edges of its tiles."""
 
 import numpy as np
 import pytest
@@ -57,6 +59,31 @@ def test_block_sizes_change_no_bits(cuda, oracle, mech, dt, ncells):
     for form in (dict(warps_per_block=1), dict(warps_per_block=4, register_budget=1), dict(warps_per_block=12)):
         y, s = _react(mech, *cells, dt, **form, **opts)
         assert np.array_equal(y, ref) and np.array_equal(s, st), form
+
+
+@pytest.mark.parametrize("mech,dt", [("LiDryer", 1e-5), ("drm19", 1e-6)])
+def test_fp32_block_sizes_change_no_bits(cuda, oracle, mech, dt):
+    cells = premix_oracle(oracle, mech, 33, 9, 1100.0, 700.0, 0.5, 1.0)
+    opts = dict(rtol=1e-10, atol=1e-10, max_order=5, lu_fp32=1)
+    ref, st = _react(mech, *cells, dt, warps_per_block=8, **opts)
+    for wpb in (1, 4, 12):
+        y, s = _react(mech, *cells, dt, warps_per_block=wpb, **opts)
+        assert np.array_equal(y, ref) and np.array_equal(s, st), wpb
+
+
+# Through ignition at rtol = 1e-10 one bit of T grows to 1e-8 of the result
+# (2-norm over the cells; ppb_bdf.cuh, UE): ten times that is the bar.
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("mech,dt", [("LiDryer", 1e-4), ("drm19", 1e-5)])
+def test_forms_of_other_roundings_agree(cuda, oracle, mech, dt, fp32):
+    cells = premix_oracle(oracle, mech, 200, 5, 1000.0, 400.0, 0.5, 1.5)
+    opts = dict(rtol=1e-10, atol=1e-10, max_order=5, lu_fp32=fp32)
+    ref, _ = _react(mech, *cells, dt, warps_per_block=8, **opts)
+    for form in (dict(warps_per_block=16), dict(warps_per_block=8, team_lanes=16),
+                 dict(warps_per_block=1, team_lanes=16)):
+        y, _ = _react(mech, *cells, dt, **form, **opts)
+        for part in (slice(0, -1), slice(-1, None)):
+            assert np.linalg.norm(y[:, part] - ref[:, part]) <= 1e-7 * np.linalg.norm(ref[:, part]), form
 
 
 def _config(mech, **opts):
