@@ -58,7 +58,7 @@ __device__ inline ArkWs ark_carve(double* p, int N, int R, int S)
 __device__ __forceinline__ void ark_f(const Team<32>& tm, const DevMech& M, int rtype, double t, const double* y,
                                       double* ydot, double rhoe, double rhoesrc, const ArkWs& w)
 {
-  reactor_rhs<32, false, NS>(tm, M, rtype, t, y, ydot, rhoe, rhoesrc, w.src, w.Y, w.sc, w.g, w.qd, w.wdot, w.ei);
+  reactor_rhs<32, false, NS, false>(tm, M, rtype, t, y, ydot, rhoe, rhoesrc, w.src, w.Y, w.sc, w.g, w.qd, w.wdot, w.ei);
 }
 
 __device__ __forceinline__ double ark_atol(const ArkParams& P, const ArkBuffers& B, int i)

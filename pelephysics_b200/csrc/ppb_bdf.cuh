@@ -153,7 +153,7 @@ __device__ __forceinline__ void rendezvous_resume(int* rv)
 // QSS: a QSS mechanism (sc and g then have its QSS slots, qco the QSS
 // solve's scratch; the team path solves the QSS concentrations only when
 // QSS is set, the one-lane path whenever the mechanism has QSS species).
-template <int TEAM, bool QSS = false, int NS = 0>
+template <int TEAM, bool QSS = false, int NS = 0, bool OUT = (NS > 16 && !QSS)>
 __device__ __forceinline__ double reactor_rhs(
   const Team<TEAM>& tm, const DevMech& M, int rtype, double t, const double* y, double* ydot, double rhoe,
   double rhoesrc, const double* src, double* Y, double* sc, double* g, double* qd, double* wdot, double* ei,
@@ -205,7 +205,7 @@ __device__ __forceinline__ double reactor_rhs(
     }
     tm.sync();
     if constexpr (QSS) qss_solve<TEAM>(tm, M, sc, g, T, invT, logT, refC, refCinv, mixture, qco, qco + 2 * M.nrq);
-    production_rate_core<TEAM, NS>(tm, M, wdot, sc, T, invT, logT, refC, refCinv, mixture, rs);
+    production_rate_core<TEAM, NS, OUT>(tm, M, wdot, sc, T, invT, logT, refC, refCinv, mixture, rs);
   } else {
     cv = mix_c(tm, M, EH, T, Y);
     for (int s = tm.lane; s < N; s += TEAM) {

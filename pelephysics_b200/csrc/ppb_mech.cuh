@@ -850,8 +850,7 @@ __device__ __forceinline__ double falloff_corr(const FoPack& f, double Corr, dou
 // as rxn_qdot).  WIDE: the mechanism has RR_WIDE reactions; they read the
 // packed record in memory.  The caller's loop is there once with and once
 // without them: one loop that asks at each reaction took 1 to 2.5 % longer in
-// mechanisms that have none (lidryer box, ReactorArkode), and out of line it
-// cost the QSS kernel 500 bytes of spills and 9 %.
+// mechanisms that have none (lidryer box, ReactorArkode).
 template <bool WIDE>
 __device__ __forceinline__ void rr_rates(const DevMech& M, const RxRate& p, int r, double T, double invT, double logT,
                                          double refC, double refCinv, double mixture, const double* sc,
@@ -1065,10 +1064,37 @@ __device__ __forceinline__ double rate_gather(const DevMech& M, int N, int s, co
   return w;
 }
 
+// production_rate_core of a mechanism with RR_WIDE reactions, out of line (the
+// temperature's terms formed again; M is a kernel's __grid_constant__ tables).
+template <int TEAM>
+__device__ __noinline__ void wide_rates(Team<TEAM> tm, const DevMech& M, double* wdot, const double* sc,
+                                        const double* g, double* qd, double T, double mixture)
+{
+  const double invT = 1.0 / T;
+  const double logT = ppb_log(T);
+  const double refC = 101325 / 8.31446 * invT;
+  const double refCinv = 1 / refC;
+  for (int r = tm.lane; r < M.nrxn; r += TEAM) {
+    const RxRate p = load_rr(M, r);
+    double qf, qr;
+    rr_rates<true>(M, p, r, T, invT, logT, refC, refCinv, mixture, sc, g, qf, qr);
+    qd[r] = __dsub_rn(qf, qr);
+  }
+  tm.sync();
+  for (int s = tm.lane; s < M.nsp; s += TEAM) wdot[s] = rate_gather(M, M.nsp, s, qd);
+  tm.sync();
+}
+
 // The reactions and the species gather of productionRate for a team of
 // lanes (TEAM > 1), given g/RT in rs.g (0 in the padding slot), sc with 1 in
 // its padding slot, and the temperature terms and mixture concentration.
-template <int TEAM, int NS = 0>
+// OUT: the rates of a mechanism with RR_WIDE reactions are out of line.  For
+// the integrators of more than 16 species that is the cheaper form for the
+// mechanisms without one (drm19 64^3 213.0 ms against 216.9 with both loops
+// inline, dodecane_lu 40.3 against 40.6); LiDryer (46.7 against 45.6), the QSS
+// kernel (500 bytes of spills, 16.3 ms against 14.9) and ReactorArkode (18.7
+// against 18.5) are better off with both inline.
+template <int TEAM, int NS = 0, bool OUT = false>
 __device__ __forceinline__ void production_rate_core(const Team<TEAM>& tm, const DevMech& M, double* wdot,
                                                      const double* sc_in, double T, double invT, double logT,
                                                      double refC, double refCinv, double mixture, RateScratch& rs)
@@ -1081,6 +1107,9 @@ __device__ __forceinline__ void production_rate_core(const Team<TEAM>& tm, const
       rr_rates<false>(M, p, r, T, invT, logT, refC, refCinv, mixture, sc_in, rs.g, qf, qr);
       rs.qd[r] = __dsub_rn(qf, qr); // both rounded: no contraction with either product
     }
+  } else if constexpr (OUT) {
+    wide_rates<TEAM>(tm, M, wdot, sc_in, rs.g, rs.qd, T, mixture);
+    return;
   } else {
     for (int r = tm.lane; r < M.nrxn; r += TEAM) {
       const RxRate p = load_rr(M, r);
