@@ -18,8 +18,8 @@ namespace ppb {
 // Newton iteration, whose residual is the FP64 right-hand side, so its
 // precision changes the convergence rate, not the converged step; the cell
 // shrinks from 8 n^2 + max(4 n^2, 40 R) to 8 n^2 + 32 R bytes plus the
-// vectors (heptane_lu_88sk: 107 KB, two cells per SM; the FP64 factor takes
-// 147 KB, one).  Nothing is added to that: the column of the row order lies
+// vectors (heptane_lu_88sk: 109,120 bytes, two cells per SM; the FP64 factor
+// takes 150,576, one).  Nothing is added to that: the column of the row order lies
 // where the row permutation is read from it, and the reciprocals of the
 // factor's diagonal where the per-reaction factors are dead until the next
 // Jacobian.  A grimech30 block of five cells has 116 bytes to spare.
